@@ -120,7 +120,7 @@ Status CsrPcg(int32_t n, const int32_t *ro, const int32_t *col, const double *va
       (s = d_r.ensure(vec)) != Status::kOk || (s = d_z.ensure(vec)) != Status::kOk ||
       (s = d_p0.ensure(vec)) != Status::kOk || (s = d_p1.ensure(vec)) != Status::kOk ||
       (s = d_q.ensure(vec)) != Status::kOk ||
-      (s = d_part.ensure(static_cast<size_t>(2) * 64 * grid_cap)) != Status::kOk ||
+      (s = d_part.ensure(fg::PcgPartialsDoubles(kp, grid_cap))) != Status::kOk ||
       (s = d_info.ensure(3 * static_cast<size_t>(kp))) != Status::kOk ||
       (s = d_bar.ensure(1)) != Status::kOk || (s = d_err.ensure(1)) != Status::kOk)
     return s;
@@ -131,6 +131,7 @@ Status CsrPcg(int32_t n, const int32_t *ro, const int32_t *col, const double *va
   a.kp = kp;
   a.items = items;
   a.slice_off = d_off.get();
+  a.host_slice_off = slice_off.data();
   a.row_len = d_len.get();
   a.sell_col = d_col.get();
   a.values = d_val.get();

@@ -62,7 +62,7 @@ struct PcgArgs {
   int32_t block_size, block_stride, block_item;
   const void *b;
   void *x, *r, *z, *p0, *p1, *q;
-  double *partials;   // [2][64][grid]
+  double *partials;   // PcgPartialsDoubles(kp, row groups)
   unsigned int *barrier;
   int32_t *error;
   double *info;       // [items][3]: status, iterations, residual
@@ -100,6 +100,10 @@ struct PcgArgs {
   // else 512), 1 CTAs of 1024 threads where the launch allows them (FP64 Jacobi, an even
   // number of row groups), 2 CTAs of 512.  Both shapes give the same bits.
   int32_t block_request;
+  // Resident form (FP64 Jacobi; pcg_resident.cuh): 0 wherever each CTA's share fits in
+  // shared memory (needs host_slice_off), 2 off.  The same bits either way.  row_groups and
+  // resident_offset are set by LaunchPcg.
+  int32_t resident_request, row_groups, resident_offset;
   // One-reduction form (FP64 Jacobi only; pcg1r_kernel.cuh): t0 / t1 are two more
   // vectors of [n_pad][kp] doubles, and partials must hold 2 x 96 x grid doubles.
   int32_t one_reduction;
@@ -134,6 +138,8 @@ cudaError_t LaunchGatherRhs(const DevicePlan &p, int kp, const double *elem_rhs,
 cudaError_t LaunchBlockInverse(const DevicePlan &p, int kp, int items, int bs, const double *values,
                                int value_item, const double *diag, int diag_item, double *out64,
                                float *out32, int32_t *fallbacks, cudaStream_t stream);
+// Whether LaunchPcg would run args in the resident form.
+bool PcgResident(const PcgArgs &args);
 // Cooperative persistent PCG; *grid_out receives the number of CTAs used.
 cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t stream);
 int PcgMaxGrid(int kp);
@@ -155,9 +161,9 @@ int MultiPcgMaxGrid(int kp = 1);
 size_t MultiPcgRingBytes(int kp);
 // Whether a PCG kernel exists for this shape (block size 32 in FP64 stops at 16 items).
 bool PcgSupported(int kp, int precision, int block_size);
-// Doubles of the partials buffer a launch of up to `grid` CTAs needs (the one-reduction
-// form reduces three sums per item).
-size_t PcgPartialsDoubles(int grid, bool one_reduction);
+// Doubles of the partials buffer a launch of up to kp items and `grid` row groups needs
+// (grows with both).
+size_t PcgPartialsDoubles(int kp, int grid);
 
 cudaError_t LaunchNewtonNorms(const DevicePlan &p, int kp, const double *x, const double *state,
                               double *partials, double *norms, cudaStream_t stream);

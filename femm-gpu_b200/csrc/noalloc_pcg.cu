@@ -229,7 +229,7 @@ Status NoallocPcg(int32_t n, const int32_t *ro, const int32_t *col, const double
   const int grid_cap = PcgMaxGrid(1);
   if (grid_cap <= 0)
     return Status::kGpuUnavailable;
-  if (grid_cap > kNoallocMaxGrid)
+  if (grid_cap > kNoallocMaxGrid || PcgPartialsDoubles(1, grid_cap) > static_cast<size_t>(2) * 64 * kNoallocMaxGrid)
     return Status::kUnsupportedFeature;
   PrepareKernel<<<1, kPrepThreads, 0, stream>>>(n, ro, col, val, diag, rhs, scratch);
   if (cudaGetLastError() != cudaSuccess)
@@ -242,6 +242,11 @@ Status NoallocPcg(int32_t n, const int32_t *ro, const int32_t *col, const double
   if (control.setup_error != kSetupOk)
     return Status::kInvalidArgument;
   const int n_pad = (n + 31) / 32 * 32;
+  int32_t slice_off[kNoallocMaxSlices + 1]; // the launch sizes its shared memory by these
+  if (cudaMemcpyAsync(slice_off, scratch + kOffSliceOff, sizeof(int32_t) * (n_pad / 32 + 1),
+                      cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+      cudaStreamSynchronize(stream) != cudaSuccess)
+    return Status::kInternalError;
   PcgArgs a{};
   a.n = n;
   a.n_pad = n_pad;
@@ -249,6 +254,7 @@ Status NoallocPcg(int32_t n, const int32_t *ro, const int32_t *col, const double
   a.kp = 1;
   a.items = 1;
   a.slice_off = reinterpret_cast<const int32_t *>(scratch + kOffSliceOff);
+  a.host_slice_off = slice_off;
   a.row_len = reinterpret_cast<const int32_t *>(scratch + kOffRowLen);
   a.sell_col = reinterpret_cast<const int32_t *>(scratch + kOffCol);
   a.values = reinterpret_cast<const double *>(scratch + kOffVal);

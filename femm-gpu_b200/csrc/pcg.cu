@@ -2,6 +2,7 @@
 // (kernel template in pcg_kernel.cuh; instantiations in pcg_f64*.cu / pcg_f32*.cu).
 #include "kernels.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -16,6 +17,9 @@ const void *PcgKernelF32Block(int kp, int bs);
 const void *MultiPcgKernelF64(int kp);
 const void *PcgKernelF64OneReduction(int kp);
 const void *PcgKernelF64Wide(int kp);
+// The resident form; *entry receives the shared-memory bytes of an operator entry of one
+// warp-step.
+const void *PcgKernelF64Resident(int kp, bool shared, int *entry);
 
 namespace
 {
@@ -133,9 +137,79 @@ int PcgMaxGrid(int kp)
   return grid;
 }
 
-size_t PcgPartialsDoubles(int grid, bool one_reduction)
+size_t PcgPartialsDoubles(int kp, int grid)
 {
-  return static_cast<size_t>(2) * (one_reduction ? 96 : 64) * static_cast<size_t>(grid);
+  // Double-buffered sums of the barrier-based reductions; the resident form's eight mailbox
+  // buffers of partials (at most 64 x 64 pairs where every CTA gets them) and result lines.
+  const size_t k = static_cast<size_t>(kp), g = static_cast<size_t>(grid);
+  const size_t partials = std::max<size_t>(2 * k * g, 2 * 64 * 64), line = std::max<size_t>(2 * k, 16);
+  return std::max<size_t>(4 * k * g + 8 * (partials + g * line), 2 * 96 * g);
+}
+
+namespace
+{
+
+// Row groups of a launch: kPcgWarps warps each, one warp-step of rows per warp at least,
+// at most the co-resident CTAs of 512 threads.
+int RowGroups(const PcgArgs &args, int max_grid)
+{
+  const int rows_per_warp = 32 * ItemsPerThread(args.kp, args.precision) / args.kp;
+  const int grid = (args.n_pad / rows_per_warp + kPcgWarps - 1) / kPcgWarps;
+  return grid > max_grid ? max_grid : (grid < 1 ? 1 : grid);
+}
+
+struct ResidentShape {
+  const void *kernel = nullptr;
+  int offset = 0;
+  size_t smem = 0;
+};
+
+// The resident form's launch (a CTA per row group), if there is an SM for every row group --
+// then no warp has more than one warp-step -- and every CTA's operator entries fit in shared
+// memory.  It is the faster form wherever it fits (pcg_resident.cuh has both sides' times).
+bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
+{
+  if (args.resident_request == 2 || args.precision != 0 || args.blocks || args.one_reduction ||
+      !args.host_slice_off)
+    return false;
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return false;
+  const int s = 32 * ItemsPerThread(args.kp, 0) / args.kp; // rows per warp-step
+  const long long ws = args.n_pad / s;
+  if (groups > sms || ws > static_cast<long long>(groups) * kPcgWarps)
+    return false;
+  long long most = 0;
+  for (int c = 0; c < groups; ++c) {
+    const long long w0 = ws * c / groups, w1 = ws * (c + 1) / groups;
+    long long entries = 0;
+    for (long long w = w0; w < w1;) { // whole slices at a time
+      const long long slice = (w * s) >> 5, end = ((slice + 1) * 32) / s;
+      const long long n = (end < w1 ? end : w1) - w;
+      entries += n * ((args.host_slice_off[slice + 1] - args.host_slice_off[slice]) / 32);
+      w += n;
+    }
+    most = entries > most ? entries : most;
+  }
+  int entry = 0;
+  const void *kernel = PcgKernelF64Resident(args.kp, args.value_item == 0, &entry);
+  const long long data = most * entry, total = data + (kPcgWarps + 1) * 4;
+  if (!kernel || total > 227 * 1024 || KernelGrid(kernel, static_cast<size_t>(total), kPcgThreads, 1) < groups)
+    return false;
+  *out = ResidentShape{kernel, static_cast<int>(data), static_cast<size_t>(total)};
+  return true;
+}
+
+} // namespace
+
+bool PcgResident(const PcgArgs &args)
+{
+  ResidentShape shape;
+  const int max_grid = PcgMaxGrid(args.kp);
+  const bool fits = max_grid > 0 && ChooseResident(args, RowGroups(args, max_grid), &shape);
+  cudaGetLastError(); // a size beyond the shared-memory limit is not an error here
+  return fits;
 }
 
 cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t stream)
@@ -157,11 +231,26 @@ cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t 
   const int iv = ItemsPerThread(args.kp, args.precision);
   const int rows_per_warp = 32 * iv / args.kp;
   const int warp_slices = args.n_pad / rows_per_warp;
-  int grid = (warp_slices + kPcgWarps - 1) / kPcgWarps; // row groups of kPcgWarps warps
-  if (grid > max_grid)
-    grid = max_grid;
-  if (grid < 1)
-    grid = 1;
+  const int grid = RowGroups(args, max_grid);
+  ResidentShape resident;
+  if (ChooseResident(args, grid, &resident)) {
+    args.row_groups = grid;
+    args.resident_offset = resident.offset;
+    cudaError_t e = cudaMemsetAsync(args.barrier, 0, sizeof(unsigned), stream);
+    if (e == cudaSuccess)
+      e = cudaMemsetAsync(args.error, 0, sizeof(int32_t), stream);
+    if (e != cudaSuccess)
+      return e;
+    void *params[] = {&args};
+    e = cudaLaunchCooperativeKernel(resident.kernel, dim3(grid), dim3(kPcgThreads), params,
+                                    resident.smem, stream);
+    if (grid_out)
+      *grid_out = grid;
+    if (block_out)
+      *block_out = kPcgThreads;
+    return e;
+  }
+  cudaGetLastError(); // a size beyond the shared-memory limit is not an error here
   // Wide CTAs (FP64 Jacobi): the same row groups two to a CTA of 1024 threads, one CTA per
   // SM -- the same rows, order and partial sums, so the same bits.
   const bool want_wide = args.block_request == 0 ? WideBlocksEnabled() : args.block_request == 1;

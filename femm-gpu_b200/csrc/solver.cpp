@@ -124,6 +124,7 @@ Status Plan::Create(HostModel model, const fg_plan_options &options)
   host_only_ = (options_.flags & FG_PLAN_HOST_ONLY) != 0;
   from_iterate_ = (options_.flags & FG_PLAN_PCG_FROM_ITERATE) != 0;
   one_reduction_ = (options_.flags & FG_PLAN_PCG_ONE_REDUCTION) != 0;
+  streamed_ = (options_.flags & FG_PLAN_PCG_STREAMED) != 0;
   if (one_reduction_ && (options_.precision != FG_PRECISION_FP64 || block_size() != 0))
     return Status::kUnsupportedFeature;
   if (host_only_)
@@ -285,7 +286,7 @@ Status Plan::EnsureWorkspace(int kp)
   FG_EN(q_, vec);
   FG_EN(norm_partials_, static_cast<size_t>(2) * kp * 256);
   FG_EN(norms_, static_cast<size_t>(2) * kp);
-  FG_EN(pcg_partials_, PcgPartialsDoubles(pcg_grid_cap_, one_reduction_));
+  FG_EN(pcg_partials_, PcgPartialsDoubles(kp, pcg_grid_cap_));
   if (one_reduction_) {
     FG_EN(t0_, vec);
     FG_EN(t1_, vec);
@@ -391,9 +392,11 @@ Status Plan::RunPcg(int kp, int items, uint32_t mask, double tolerance, int max_
 
 namespace
 {
-// CG iterations of each timed candidate launch, and rounds over the candidates.
+// CG iterations of each timed candidate launch, and rounds over the candidates.  Where the
+// resident form runs instead of them, one short round reports their times.
 constexpr int kTuneIterations = 64;
 constexpr int kTuneRounds = 2;
+constexpr int kTuneIterationsResident = 16;
 
 bool TuningEnabled()
 {
@@ -404,7 +407,8 @@ bool TuningEnabled()
 
 cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t stream)
 {
-  const int key = a.kp * 1000 + a.precision * 100 + (a.blocks ? a.block_size : 0);
+  const int key = a.kp * 1000 + a.precision * 100 + (a.blocks ? a.block_size : 0) + (a.value_item ? 0 : 100000);
+  a.resident_request = streamed_ ? 2 : 0;
   auto it = shapes_.find(key);
   if (it == shapes_.end() && TuningEnabled()) {
     fg_pcg_shape sh{};
@@ -427,17 +431,21 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     }
     // One untimed launch first (cold caches and clocks would favour whichever candidate
     // runs later), then kTuneRounds interleaved rounds; each candidate keeps its fastest.
+    const bool resident = PcgResident(a);
+    const int iterations = resident ? kTuneIterationsResident : kTuneIterations;
+    const int rounds = resident ? 1 : kTuneRounds;
     PcgArgs t = a;
     t.tolerance = 0.0;
     t.item_tolerance = nullptr;
-    t.max_iterations = kTuneIterations;
+    t.max_iterations = iterations;
     t.trace = nullptr;
     t.block_request = 2;
+    t.resident_request = 2;
     if (LaunchPcg(t, nullptr, nullptr, stream) != cudaSuccess)
       cudaGetLastError();
     else
       timing_.kernel_launches += 1;
-    for (int round = 0; round < kTuneRounds; ++round)
+    for (int round = 0; round < rounds; ++round)
       for (int c = 0; c < 5; ++c) {
         const int ring = c % 2 == 0 ? 1 : 2, cache = c == 2 || c == 3 ? 1 : 2;
         if (ring == 1 && !ring_possible)
@@ -456,7 +464,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         timing_.kernel_launches += 1;
         if (c == 4 && threads != 1024)
           continue; // the launch fell back to 512 threads: not a candidate of its own
-        const double us = 1e3 * ms / kTuneIterations;
+        const double us = 1e3 * ms / iterations;
         if (sh.us_per_iteration[c] == 0.0) {
           ++sh.candidates;
           sh.us_per_iteration[c] = us;
@@ -472,6 +480,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         sh.column_cache = c == 2 || c == 3 ? 1 : 0;
         sh.threads_per_block = c == 4 ? 1024 : 512;
       }
+    sh.resident = resident ? 1 : 0;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (sh.candidates > 0)
@@ -481,6 +490,8 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     a.ring_request = it->second.value_ring ? 1 : 2;
     a.col_cache_request = it->second.column_cache ? 1 : 2;
     a.block_request = it->second.threads_per_block == 1024 ? 1 : 2;
+    if (!it->second.resident)
+      a.resident_request = 2;
   }
   return LaunchPcg(a, grid, block, stream);
 }
@@ -792,6 +803,7 @@ Status Plan::EnsureLanes(int lanes)
     lane->options_.flags |= FG_PLAN_HOST_ONLY;
     lane->chunk_cap_ = chunk_cap_;
     lane->from_iterate_ = from_iterate_;
+    lane->streamed_ = streamed_;
     lane->host_only_ = true;
     Status s = lane->AttachDevice();
     if (s != Status::kOk)

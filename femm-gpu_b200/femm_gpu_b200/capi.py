@@ -33,6 +33,7 @@ STATUS_NAMES = [
 PLAN_HOST_ONLY = 1
 PLAN_PCG_FROM_ITERATE = 2
 PLAN_PCG_ONE_REDUCTION = 4
+PLAN_PCG_STREAMED = 8
 
 EXPORTED = [
     "fg_production_options", "fg_status_name", "fg_abi_version", "fg_plan_create",
@@ -140,7 +141,7 @@ class FgPcgShape(C.Structure):
     _fields_ = [("items", C.c_int32), ("precision", C.c_int32), ("block_size", C.c_int32),
                 ("value_ring", C.c_int32), ("column_cache", C.c_int32), ("candidates", C.c_int32),
                 ("us_per_iteration", C.c_double * 5), ("threads_per_block", C.c_int32),
-                ("reserved", C.c_int32)]
+                ("resident", C.c_int32)]
 
 
 _LIB = None
@@ -217,7 +218,7 @@ class Plan:
 
     def __init__(self, model: Model, preconditioner: int = 0, block_size: int = 8,
                  precision: int = 0, host_only: bool = False, from_iterate: bool = False,
-                 one_reduction: bool = False):
+                 one_reduction: bool = False, streamed: bool = False):
         self.model = model
         L = lib()
         self._keep = []
@@ -247,7 +248,7 @@ class Plan:
             self._keep.append(ages)
             fm.air_gap_count, fm.air_gap_elements = len(model.ages), C.cast(ages, C.c_void_p)
         flags = ((PLAN_HOST_ONLY if host_only else 0) | (PLAN_PCG_FROM_ITERATE if from_iterate else 0) |
-                 (PLAN_PCG_ONE_REDUCTION if one_reduction else 0))
+                 (PLAN_PCG_ONE_REDUCTION if one_reduction else 0) | (PLAN_PCG_STREAMED if streamed else 0))
         opts = FgPlanOptions(preconditioner, block_size, precision, flags)
         self._h = C.c_void_p()
         status = L.fg_plan_create(C.byref(fm), C.byref(opts), C.byref(self._h))
@@ -440,7 +441,7 @@ class Plan:
         return [{"items": a.items, "precision": a.precision, "block_size": a.block_size,
                  "value_ring": bool(a.value_ring), "column_cache": bool(a.column_cache),
                  "candidates": a.candidates, "us_per_iteration": list(a.us_per_iteration),
-                 "threads_per_block": a.threads_per_block}
+                 "threads_per_block": a.threads_per_block, "resident": bool(a.resident)}
                 for a in arr[:n]]
 
 

@@ -138,7 +138,14 @@ typedef struct fg_plan_options {
  * (the true-residual check); results agree with the default form within the solve's
  * tolerance, not bit for bit.  With block-Jacobi or mixed precision fg_plan_create
  * returns FG_UNSUPPORTED_FEATURE. */
-enum { FG_PLAN_HOST_ONLY = 1, FG_PLAN_PCG_FROM_ITERATE = 2, FG_PLAN_PCG_ONE_REDUCTION = 4 };
+/* FG_PLAN_PCG_STREAMED: the plan's PCG launches never keep their share of the system in
+ * shared memory (the resident form, chosen where it fits); same results bit for bit. */
+enum {
+  FG_PLAN_HOST_ONLY = 1,
+  FG_PLAN_PCG_FROM_ITERATE = 2,
+  FG_PLAN_PCG_ONE_REDUCTION = 4,
+  FG_PLAN_PCG_STREAMED = 8
+};
 
 /* NonlinearOptions (gpu_solver/src/physics/nonlinear_model.h:102-109). */
 typedef struct fg_solve_options {
@@ -356,8 +363,8 @@ typedef struct fg_pcg_shape {
    * CTAs (two row groups each, FP64 Jacobi with an even number of row groups), ring on,
    * cache off; 0 if not timed */
   double us_per_iteration[5];
-  int32_t threads_per_block; /* the chosen CTA shape: 512 or 1024 (the same bits either way) */
-  int32_t reserved;
+  int32_t threads_per_block; /* the fastest of these: 512 or 1024 (the same bits either way) */
+  int32_t resident;          /* 1: the resident form (not among these) was faster and is used */
 } fg_pcg_shape;
 int fg_plan_pcg_shapes(const fg_plan *plan, int32_t capacity, fg_pcg_shape *shapes);
 
