@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <vector>
 
 namespace fg
 {
@@ -20,6 +21,10 @@ const void *PcgKernelF64Wide(int kp);
 // The resident form; *entry receives the shared-memory bytes of an operator entry of one
 // warp-step.
 const void *PcgKernelF64Resident(int kp, bool shared, int *entry);
+// The same for several warp-steps per warp: `groups` (1 or 2) row groups per CTA, stream:
+// values read from L2 (always with one); *step receives the bytes of a warp-step besides its
+// entries.
+const void *PcgKernelF64ResidentSteps(int kp, bool shared, bool stream, int groups, int *step, int *entry);
 
 namespace
 {
@@ -160,13 +165,14 @@ int RowGroups(const PcgArgs &args, int max_grid)
 
 struct ResidentShape {
   const void *kernel = nullptr;
-  int offset = 0;
+  int ctas = 0, offset = 0;
   size_t smem = 0;
 };
 
-// The resident form's launch (a CTA per row group), if there is an SM for every row group --
-// then no warp has more than one warp-step -- and every CTA's operator entries fit in shared
-// memory.  It is the faster form wherever it fits (pcg_resident.cuh has both sides' times).
+// The resident form's launch, if the CTAs' shares fit in shared memory.  With an SM for every
+// row group no warp has more than one warp-step and the state sits in registers (if the
+// entries fit; wide rows may not); else a CTA has two row groups and the state sits in shared
+// memory, the operator's values beside it or, where they do not fit, in L2.
 bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
 {
   if (args.resident_request == 2 || args.precision != 0 || args.blocks || args.one_reduction ||
@@ -178,27 +184,50 @@ bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
     return false;
   const int s = 32 * ItemsPerThread(args.kp, 0) / args.kp; // rows per warp-step
   const long long ws = args.n_pad / s;
-  if (groups > sms || ws > static_cast<long long>(groups) * kPcgWarps)
+  const bool shared = args.value_item == 0;
+  const int per_cta = groups <= sms ? 1 : 2, ctas = (groups + per_cta - 1) / per_cta;
+  // The least a CTA can need with the state in shared memory, before looking at the rows.
+  int step = 0, entry = 0;
+  if (!PcgKernelF64ResidentSteps(args.kp, shared, true, per_cta, &step, &entry) ||
+      (ws / ctas) * (step + entry) > 227 * 1024)
     return false;
-  long long most = 0;
-  for (int c = 0; c < groups; ++c) {
-    const long long w0 = ws * c / groups, w1 = ws * (c + 1) / groups;
-    long long entries = 0;
+  // Steps and operator entries of every CTA.
+  std::vector<long long> steps(ctas), entries(ctas);
+  for (int c = 0; c < ctas; ++c) {
+    const long long w0 = ws * (c * per_cta) / groups, w1 = ws * std::min(groups, (c + 1) * per_cta) / groups;
+    steps[c] = w1 - w0;
     for (long long w = w0; w < w1;) { // whole slices at a time
       const long long slice = (w * s) >> 5, end = ((slice + 1) * 32) / s;
       const long long n = (end < w1 ? end : w1) - w;
-      entries += n * ((args.host_slice_off[slice + 1] - args.host_slice_off[slice]) / 32);
+      entries[c] += n * ((args.host_slice_off[slice + 1] - args.host_slice_off[slice]) / 32);
       w += n;
     }
-    most = entries > most ? entries : most;
   }
-  int entry = 0;
-  const void *kernel = PcgKernelF64Resident(args.kp, args.value_item == 0, &entry);
-  const long long data = most * entry, total = data + (kPcgWarps + 1) * 4;
-  if (!kernel || total > 227 * 1024 || KernelGrid(kernel, static_cast<size_t>(total), kPcgThreads, 1) < groups)
-    return false;
-  *out = ResidentShape{kernel, static_cast<int>(data), static_cast<size_t>(total)};
-  return true;
+  auto fits = [&](const void *kernel, long long step_bytes, long long entry_bytes) {
+    long long data = 0, most = 0;
+    for (int c = 0; c < ctas; ++c) {
+      data = std::max(data, steps[c] * step_bytes + entries[c] * entry_bytes);
+      most = std::max(most, steps[c]);
+    }
+    const long long total = data + (most + 1) * 4;
+    if (!kernel || total > 227 * 1024 || KernelGrid(kernel, static_cast<size_t>(total), kPcgThreads, 1) < ctas)
+      return false;
+    *out = ResidentShape{kernel, ctas, static_cast<int>(data), static_cast<size_t>(total)};
+    return true;
+  };
+  if (per_cta == 1 && ws <= static_cast<long long>(groups) * kPcgWarps) {
+    const void *kernel = PcgKernelF64Resident(args.kp, shared, &entry);
+    if (fits(kernel, 0, entry))
+      return true;
+  }
+  for (const bool stream : {false, true}) {
+    if (!stream && per_cta == 1)
+      continue;
+    const void *kernel = PcgKernelF64ResidentSteps(args.kp, shared, stream, per_cta, &step, &entry);
+    if (fits(kernel, step, entry))
+      return true;
+  }
+  return false;
 }
 
 } // namespace
@@ -242,10 +271,10 @@ cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t 
     if (e != cudaSuccess)
       return e;
     void *params[] = {&args};
-    e = cudaLaunchCooperativeKernel(resident.kernel, dim3(grid), dim3(kPcgThreads), params,
+    e = cudaLaunchCooperativeKernel(resident.kernel, dim3(resident.ctas), dim3(kPcgThreads), params,
                                     resident.smem, stream);
     if (grid_out)
-      *grid_out = grid;
+      *grid_out = resident.ctas;
     if (block_out)
       *block_out = kPcgThreads;
     return e;

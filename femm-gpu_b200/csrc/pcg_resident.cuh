@@ -87,8 +87,9 @@ template <int ID> __device__ __forceinline__ void NamedSync()
   asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(kPcgThreads) : "memory");
 }
 
-template <int KP> struct ResidentShared {
-  double warp[kPcgWarps][2 * KP]; // the warps' sums
+// GV: row groups per CTA.
+template <int KP, int GV> struct ResidentShared {
+  double warp[kPcgWarps * GV][2 * KP]; // the warps' sums, row group by row group
   int err;    // GridBarrier's
   int failed; // a wait for a message ran out
   // What the CTA goes on with after a reduction: the active items, and kStop (a wait ran out)
@@ -113,12 +114,13 @@ __device__ __forceinline__ bool PollAgain(const PcgArgs &a, unsigned &spin, unsi
   return false;
 }
 
-// A warp's part of Q per-item sums (or maxima).
-template <int KP, int IV, int Q, bool kMax>
-__device__ __forceinline__ void WarpPart(double (&v)[Q][IV], ResidentShared<KP> &sm)
+// A warp's part of Q per-item sums (or maxima); place: row group in the CTA x kPcgWarps + the
+// group's warp whose rows they are.
+template <int KP, int IV, int GV, int Q, bool kMax>
+__device__ __forceinline__ void WarpPart(double (&v)[Q][IV], int place, ResidentShared<KP, GV> &sm)
 {
   constexpr int LR = KP / IV;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int off = 16; off >= LR; off >>= 1)
 #pragma unroll
@@ -133,7 +135,7 @@ __device__ __forceinline__ void WarpPart(double (&v)[Q][IV], ResidentShared<KP> 
     for (int q = 0; q < Q; ++q)
 #pragma unroll
       for (int j = 0; j < IV; ++j)
-        sm.warp[warp][q * KP + lane * IV + j] = v[q][j];
+        sm.warp[place][q * KP + lane * IV + j] = v[q][j];
 }
 
 // The mailboxes behind a.partials: after the two buffers of the barrier-based reductions
@@ -144,20 +146,21 @@ __device__ __forceinline__ void WarpPart(double (&v)[Q][IV], ResidentShared<KP> 
 // results: every CTA reads all partials.
 template <int KP> struct Mailboxes {
   double *base;
-  int G, padded; // row groups = CTAs, and rounded up to a power of two
+  int G, ctas, padded; // row groups, CTAs, row groups rounded up to a power of two
   bool direct;
   unsigned results, stride; // doubles before a buffer's results, and of a whole buffer
   static constexpr int kLine = 2 * KP > 16 ? 2 * KP : 16;
-  __device__ __forceinline__ void Init(const PcgArgs &a)
+  __device__ __forceinline__ void Init(const PcgArgs &a, int ctas_)
   {
+    ctas = ctas_;
     base = a.partials + static_cast<size_t>(2) * 2 * KP * a.row_groups;
     G = a.row_groups;
     padded = 1;
     while (padded < G)
       padded <<= 1;
-    direct = KP * padded <= kDirect;
+    direct = ctas == G && KP * padded <= kDirect;
     results = static_cast<unsigned>(KP * G * 2);
-    stride = results + static_cast<unsigned>(G * kLine);
+    stride = results + static_cast<unsigned>(ctas * kLine);
   }
   __device__ __forceinline__ double *Buffer(int r) const
   {
@@ -174,7 +177,7 @@ template <int KP> struct Mailboxes {
       for (int it = t; it < KP; it += n)
         StoreMessage<2>(Partial(r, it, c), unset);
     } else {
-      for (int it = c; it < KP; it += G)
+      for (int it = c; it < KP; it += ctas)
         for (int g = t; g < G; g += n)
           StoreMessage<2>(Partial(r, it, g), unset);
       for (int it = t; it < KP; it += n)
@@ -211,34 +214,34 @@ __device__ __forceinline__ void Poll(const PcgArgs &a, const double *base, int s
 // Warp 0's half of a CG loop reduction of Q per-item sums, in GridReduce's order: the lanes
 // of a warp (WarpPart), the 16 warps of a row group, then the row groups lane-strided over
 // one warp.  First it sends the CTA's partials ...
-template <int KP, int Q>
-__device__ __forceinline__ void SendPartials(int rank, const Mailboxes<KP> &mail, ResidentShared<KP> &sm, int r)
+template <int KP, int GV, int Q>
+__device__ __forceinline__ void SendPartials(int rank, const Mailboxes<KP> &mail, ResidentShared<KP, GV> &sm, int r)
 {
   constexpr int QK = Q * KP;
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int t0 = 0; t0 < QK; t0 += 32) {
-    const int t = t0 + lane;
-    if (t < QK) {
+  for (int t0 = 0; t0 < QK * GV; t0 += 32) {
+    const int gv = (t0 + lane) / QK, t = (t0 + lane) % QK;
+    if (gv < GV && rank * GV + gv < mail.G) {
       double w[kPcgWarps];
 #pragma unroll
       for (int i = 0; i < kPcgWarps; ++i)
-        w[i] = sm.warp[i][t];
+        w[i] = sm.warp[gv * kPcgWarps + i][t];
       double s = w[0];
 #pragma unroll
       for (int i = 1; i < kPcgWarps; ++i)
         s += w[i];
       const double m[1] = {Sendable(s)};
-      StoreMessage<1>(mail.Partial(r, t % KP, rank) + t / KP, m);
+      StoreMessage<1>(mail.Partial(r, t % KP, rank * GV + gv) + t / KP, m);
     }
   }
 }
 
 // ... then it sums the items this CTA owns and sends their results to every CTA (or sums
 // every item itself, direct).  Lane `item` leaves with the item's sums.
-template <int KP, int Q>
+template <int KP, int GV, int Q>
 __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailboxes<KP> &mail,
-                                        ResidentShared<KP> &sm, int r, double (&sum)[Q])
+                                        ResidentShared<KP, GV> &sm, int r, double (&sum)[Q])
 {
   const int lane = threadIdx.x & 31, G = mail.G;
   if (mail.direct) {
@@ -275,7 +278,7 @@ __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailbo
     }
     return;
   }
-  for (int it = rank; it < KP; it += G) {
+  for (int it = rank; it < KP; it += mail.ctas) {
     double s[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q)
@@ -299,7 +302,7 @@ __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailbo
       for (int q = 0; q < Q; ++q)
         s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
     const double m[2] = {Sendable(s[0]), Sendable(s[Q - 1])};
-    for (int c = lane; c < G; c += 32)
+    for (int c = lane; c < mail.ctas; c += 32)
       StoreMessage<2>(mail.Result(r, c, it), m);
   }
   double y[1][2];
@@ -311,22 +314,23 @@ __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailbo
 
 // The same sums in the rare phases (set-up, verification, the end of the budget), behind a
 // full grid barrier: every CTA's stores before it are seen by every CTA after it.
-template <int KP, int Q, bool kMax, class F>
-__device__ __forceinline__ bool BarrierReduce(const PcgArgs &a, int rank, int G,
-                                              ResidentShared<KP> &sm, unsigned &epoch, int &buf, F control)
+template <int KP, int GV, int Q, bool kMax, class F>
+__device__ __forceinline__ bool BarrierReduce(const PcgArgs &a, int rank, int ctas, int G, ResidentShared<KP, GV> &sm,
+                                              unsigned &epoch, int &buf, F control)
 {
   constexpr int QK = Q * KP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *part = a.partials + static_cast<size_t>(buf) * 2 * KP * G;
   __syncthreads();
-  if (threadIdx.x < QK) {
-    const int t = threadIdx.x;
-    double s = sm.warp[0][t];
+  if (threadIdx.x < QK * GV) {
+    const int gv = static_cast<int>(threadIdx.x) / QK, t = static_cast<int>(threadIdx.x) % QK;
+    double s = sm.warp[gv * kPcgWarps][t];
     for (int i = 1; i < kPcgWarps; ++i)
-      s = kMax ? fmax(s, sm.warp[i][t]) : s + sm.warp[i][t];
-    part[static_cast<size_t>(t) * G + rank] = s;
+      s = kMax ? fmax(s, sm.warp[gv * kPcgWarps + i][t]) : s + sm.warp[gv * kPcgWarps + i][t];
+    if (rank * GV + gv < G)
+      part[static_cast<size_t>(t) * G + rank * GV + gv] = s;
   }
-  if (!GridBarrier(a, GridShape{G, rank}, epoch, sm))
+  if (!GridBarrier(a, GridShape{ctas, rank}, epoch, sm))
     return false;
   for (int it = warp; it < KP; it += kPcgWarps) {
     double s[Q];
@@ -366,7 +370,7 @@ template <int KP, int IV, bool SHARED> struct ResidentLayout {
 template <int KP, int IV, bool SHARED>
 __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
 {
-  __shared__ ResidentShared<KP> sm;
+  __shared__ ResidentShared<KP, 1> sm;
   __shared__ Control ctl;
   __shared__ Trace tr;
   __shared__ Mailboxes<KP> mail;
@@ -419,7 +423,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
       tr.slot[s] = 0;
     tr.mark = GlobalTimer();
     sm.err = sm.failed = 0;
-    mail.Init(a);
+    mail.Init(a, G);
   }
   __syncthreads();
   // The mailboxes start unset; the set-up's barriers make that known.
@@ -512,8 +516,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
           v[1][j] = fmax(v[1][j], fabs(bj));
         }
     }
-    WarpPart<KP, IV, 2, true>(v, sm);
-    if (!BarrierReduce<KP, 2, true>(a, rank, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
+    WarpPart<KP, IV, 1, 2, true>(v, warp, sm);
+    if (!BarrierReduce<KP, 1, 2, true>(a, rank, G, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
           if (!ctl.active[it])
             return;
           const double pr = sum[0];
@@ -554,8 +558,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
           v[1][j] += rv[j] * zv[j];
         }
     }
-    WarpPart<KP, IV, 2, false>(v, sm);
-    if (!BarrierReduce<KP, 2, false>(a, rank, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
+    WarpPart<KP, IV, 1, 2, false>(v, warp, sm);
+    if (!BarrierReduce<KP, 1, 2, false>(a, rank, G, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
           if (!ctl.active[it])
             return;
           const double rr = sum[0], rho = sum[1];
@@ -698,17 +702,17 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
           v[0][j] = pv[j] * qv[j];
         }
       }
-      WarpPart<KP, IV, 1, false>(v, sm);
+      WarpPart<KP, IV, 1, 1, false>(v, warp, sm);
     }
     if (warp == 0) {
       const int it = lane < KP ? lane : 0;
       const double rho = ctl.rho[it];
       NamedSync<1>();
       mark(0);
-      SendPartials<KP, 1>(rank, mail, sm, red);
+      SendPartials<KP, 1, 1>(rank, mail, sm, red);
       FenceAcqRel();
       double sum[1];
-      Collect<KP, 1>(a, rank, mail, sm, red, sum);
+      Collect<KP, 1, 1>(a, rank, mail, sm, red, sum);
       if (lane < KP && ((active >> lane) & 1u)) {
         const double pq = sum[0];
         if (pq > 0.0 && rho > 0.0 && isfinite(pq) && isfinite(rho)) {
@@ -752,7 +756,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
           v[1][j] = rv[j] * zv[j];
         }
       }
-      WarpPart<KP, IV, 2, false>(v, sm);
+      WarpPart<KP, IV, 1, 2, false>(v, warp, sm);
     }
     // While the sums travel: gather the z of the next phase A, reset the z of this iteration
     // (every CTA's phase A of it is over: the buffer serves iteration + 4) and the mailboxes
@@ -763,13 +767,13 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
       const double rho = ctl.rho[it], thr = ctl.thr[it];
       NamedSync<1>();
       mark(2);
-      SendPartials<KP, 2>(rank, mail, sm, red);
+      SendPartials<KP, 1, 2>(rank, mail, sm, red);
       if (mine) {
         fetch(zn);
         reset_z(z);
       }
       double sum[2];
-      Collect<KP, 2>(a, rank, mail, sm, red, sum);
+      Collect<KP, 1, 2>(a, rank, mail, sm, red, sum);
       bool at = false;
       if (lane < KP) {
         ctl.flag[it] = 0;
@@ -839,8 +843,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
               v[0][j] = t[j] * t[j];
             }
         }
-        WarpPart<KP, IV, 1, false>(v, sm);
-        if (!BarrierReduce<KP, 1, false>(a, rank, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
+        WarpPart<KP, IV, 1, 1, false>(v, warp, sm);
+        if (!BarrierReduce<KP, 1, 1, false>(a, rank, G, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
               if (!ctl.active[it] || ctl.flag[it] != 1)
                 return;
               const double trr = sum[0];
@@ -875,8 +879,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
         if (restart) // items that go on keep r, so their z is the same product again
           send_z(zn, zv);
       }
-      WarpPart<KP, IV, 2, false>(v, sm);
-      if (!BarrierReduce<KP, 2, false>(a, rank, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
+      WarpPart<KP, IV, 1, 2, false>(v, warp, sm);
+      if (!BarrierReduce<KP, 1, 2, false>(a, rank, G, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
             if (!ctl.active[it])
               return;
             if (ctl.flag[it] == 2) {
@@ -921,8 +925,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
           if (on(j))
             v[0][j] = t[j] * t[j];
       }
-      WarpPart<KP, IV, 1, false>(v, sm);
-      if (!BarrierReduce<KP, 1, false>(a, rank, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
+      WarpPart<KP, IV, 1, 1, false>(v, warp, sm);
+      if (!BarrierReduce<KP, 1, 1, false>(a, rank, G, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
             if (!ctl.active[it])
               return;
             const double trr = sum[0];
@@ -943,8 +947,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentKernel(PcgArgs a)
         if (!isfinite(x[j]))
           v[0][j] = 1.0;
       }
-    WarpPart<KP, IV, 1, false>(v, sm);
-    if (!BarrierReduce<KP, 1, false>(a, rank, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
+    WarpPart<KP, IV, 1, 1, false>(v, warp, sm);
+    if (!BarrierReduce<KP, 1, 1, false>(a, rank, G, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
           if (!ctl.active[it])
             return;
           if (sum[0] != 0.0) {

@@ -2,8 +2,9 @@
 exchanging messages) against the streamed form: the same partition, operations and summation
 orders, so the same bits -- iterates, residuals, iteration counts and statuses.  The sizes
 sit at the edges of the form: less than one row group, two, the last one with a row group per
-SM and the first without, one row group per warp-step width, and rows wider than the eight
-entries gathered ahead."""
+SM and the first without (two row groups per CTA, an odd number of them, the operator's values
+in shared memory or in L2, several steps per warp), and rows wider than the eight entries
+gathered together."""
 import numpy as np
 import pytest
 
@@ -30,7 +31,8 @@ def solve_both(model, items, limit=15.0, **options):
 
 
 @pytest.mark.parametrize("m, items", [(4, 1), (23, 1), (24, 1), (24, 3), (46, 2), (64, 4), (65, 7), (64, 16),
-                                      (65, 32), (138, 8), (139, 8)])
+                                      (65, 32), (138, 8), (139, 8),
+                                      (250, 4), (100, 32), (130, 16), (390, 1), (270, 2)])
 def test_squares_give_the_streamed_bits(gpu, m, items):
     r = solve_both(meshes.square_nonlinear(m=m, seed=3), items)
     assert all(s == 0 for s in r.status)
@@ -41,6 +43,12 @@ def test_squares_give_the_streamed_bits(gpu, m, items):
                          ids=["antiperiodic", "axisymmetric", "wide_rows"])
 def test_other_models_give_the_streamed_bits(gpu, model):
     assert all(s == 0 for s in solve_both(model, 3).status)
+
+
+def test_wide_rows_that_leave_the_values_in_l2(gpu):
+    """One row group per CTA whose entries do not fit beside the state: 20-entry ring rows."""
+    r = solve_both(meshes.sliding_band_machine(80, 60), 8, max_newton_iterations=3, recover_nonconvergence=0)
+    assert all(i.linear_iterations > 100 for i in r.info)
 
 
 def test_exhausted_budget_and_inactive_items(gpu):
