@@ -8,9 +8,11 @@
 // reproducible for a given seed.
 //
 // Kernels: one tiled FP32 GEMM with arbitrary operand strides serves the forward pass
-// (bias + GELU fused into its epilogue, pre-activations kept for the backward pass), the
-// weight gradients (A^T B shapes) and the back-propagated deltas (GELU' fused); column
-// sums give bias gradients; one elementwise kernel applies Adam.  GELU is the exact
+// (bias + GELU fused into its epilogue, pre-activations kept for the backward pass; in the
+// output layer also the loss and its delta), the weight gradients (A^T B shapes, bias
+// gradients as row sums of A) and the back-propagated deltas (GELU' fused).  A layer's weight
+// gradient and the delta below it depend on the same delta, so they share a launch: a
+// training step is six launches, two gathers and Adam.  One elementwise kernel applies Adam.  GELU is the exact
 // erf form, 0.5 x (1 + erf(x / sqrt 2)).
 #include "mlp.h"
 
@@ -24,11 +26,14 @@ namespace fg
 namespace
 {
 
-constexpr int kTile = 32;    // GEMM output tile (kTile x kTile) per 256-thread CTA
-constexpr int kTileK = 16;   // inner-dimension slab staged in shared memory
+constexpr int kTileM = 16, kTileN = 32;  // output tile of a CTA
+constexpr int kGemmThreads = 512, kGemmWarps = kGemmThreads / 32;
+constexpr int kWarpK = 16, kSlab = kGemmWarps * kWarpK; // inner dimension per warp and staged at a time
+constexpr int kPitchA = kTileM + 4, kPitchB = kTileN + 4; // floats of a staged k (16-byte rows)
+constexpr size_t kGemmSmem = sizeof(float) * kSlab * (kPitchA + kPitchB);
 constexpr int kThreads = 256;
 
-enum Epilogue : int { kStore = 0, kBiasGelu = 1, kBias = 2, kGeluGrad = 3 };
+enum Epilogue : int { kStore = 0, kBiasGelu = 1, kBias = 2, kGeluGrad = 3, kBiasDelta = 4 };
 
 __device__ __forceinline__ float Gelu(float x)
 {
@@ -44,97 +49,198 @@ __device__ __forceinline__ float GeluGrad(float x)
 // C(m, n) = epilogue(sum_k A(m, k) B(k, n)), A(m, k) = A[m * am + k * ak],
 // B(k, n) = B[k * bk + n * bn], C row-major with leading dimension ldc.
 // kBiasGelu: pre = acc + bias[n] -> aux(m, n) = pre, C = GELU(pre);  kBias: C = acc + bias[n];
-// kGeluGrad: C = acc * GELU'(aux(m, n)).
-__global__ void __launch_bounds__(kThreads)
-    GemmKernel(int M, int N, int K, const float *__restrict__ A, int am, int ak,
-               const float *__restrict__ B, int bk, int bn, float *__restrict__ C, int ldc,
-               int epilogue, const float *__restrict__ bias, float *__restrict__ aux)
+// kGeluGrad: C = acc * GELU'(aux(m, n));  kBiasDelta: C = y = acc + bias[n] and, for the
+// target t, delta = (y - t) / M and the tile's sum of 0.5 (y - t)^2 in loss[tile].
+// row_sum (optional): row_sum[m] = sum_k A(m, k).
+struct GemmArgs {
+  int M, N, K;
+  const float *A;
+  int am, ak;
+  const float *B;
+  int bk, bn;
+  float *C;
+  int ldc, epilogue;
+  const float *bias;
+  float *aux;
+  const float *target;
+  float *delta, *loss, *row_sum;
+  int tiles_n, tiles; // set by the launch
+};
+
+// Stages X(r, k) = X[r * rs + k * ks], r0 <= r < r0 + ROWS, a slab from k0 on, as
+// smem[k][r], zero outside; 16-byte loads along the contiguous direction where aligned.
+template <int ROWS, int PITCH>
+__device__ __forceinline__ void Stage(float *smem, const float *X, int rs, int ks, int r0, int rows, int k0, int K)
 {
-  __shared__ float As[kTileK][kTile + 1];
-  __shared__ float Bs[kTileK][kTile + 1];
-  const int tx = threadIdx.x % kTile, ty = threadIdx.x / kTile; // ty in [0, 8)
-  const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < K; k0 += kTileK) {
-    for (int t = threadIdx.x; t < kTileK * kTile; t += kThreads) {
-      const int kk = t / kTile, mm = t % kTile;
-      const int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < M && k < K) ? A[static_cast<size_t>(m) * am + static_cast<size_t>(k) * ak] : 0.f;
-      const int n = n0 + mm;
-      Bs[kk][mm] = (n < N && k < K) ? B[static_cast<size_t>(k) * bk + static_cast<size_t>(n) * bn] : 0.f;
+  const int slab = min(kSlab, (K - k0 + kWarpK - 1) / kWarpK * kWarpK);
+  const bool aligned = (reinterpret_cast<size_t>(X) & 15) == 0;
+  if (rs == 1 && ks % 4 == 0 && aligned) {
+    for (int t = threadIdx.x; t < slab * (ROWS / 4); t += kGemmThreads) {
+      const int k = t / (ROWS / 4), r = t % (ROWS / 4) * 4;
+      const float *x = X + static_cast<size_t>(k0 + k) * ks + r0 + r;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k0 + k < K) {
+        if (r0 + r + 3 < rows) {
+          v = *reinterpret_cast<const float4 *>(x);
+        } else {
+          v.x = r0 + r < rows ? x[0] : 0.f;
+          v.y = r0 + r + 1 < rows ? x[1] : 0.f;
+          v.z = r0 + r + 2 < rows ? x[2] : 0.f;
+        }
+      }
+      *reinterpret_cast<float4 *>(smem + k * PITCH + r) = v;
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kTileK; ++kk) {
-      const float b = Bs[kk][tx];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        acc[i] = fmaf(As[kk][ty + 8 * i], b, acc[i]);
+  } else if (ks == 1 && rs % 4 == 0 && aligned) {
+    for (int t = threadIdx.x; t < slab / 4 * ROWS; t += kGemmThreads) {
+      const int k = t / ROWS * 4, r = t % ROWS;
+      const float *x = X + static_cast<size_t>(r0 + r) * rs + k0 + k;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r0 + r < rows) {
+        if (k0 + k + 3 < K) {
+          v = *reinterpret_cast<const float4 *>(x);
+        } else {
+          v.x = k0 + k < K ? x[0] : 0.f;
+          v.y = k0 + k + 1 < K ? x[1] : 0.f;
+          v.z = k0 + k + 2 < K ? x[2] : 0.f;
+        }
+      }
+      smem[k * PITCH + r] = v.x;
+      smem[(k + 1) * PITCH + r] = v.y;
+      smem[(k + 2) * PITCH + r] = v.z;
+      smem[(k + 3) * PITCH + r] = v.w;
     }
-    __syncthreads();
+  } else {
+    for (int t = threadIdx.x; t < slab * ROWS; t += kGemmThreads) {
+      const int k = t / ROWS, r = t % ROWS;
+      smem[k * PITCH + r] = r0 + r < rows && k0 + k < K
+                                ? X[static_cast<size_t>(r0 + r) * rs + static_cast<size_t>(k0 + k) * ks]
+                                : 0.f;
+    }
   }
-  const int n = n0 + tx;
-  if (n >= N)
+}
+
+// One or two independent products per launch: CTA b computes tile b of g, or tile
+// b - g.tiles of h; with `loss`, one CTA more sums `count` loss partials.
+//
+// These products are small (256 x 256 x 256 is 34 MFLOP): latency bounds them -- of the
+// launch, of L2 and of each thread's chain -- not FP32 rate.  16 x 32 tiles give a 256 x 256
+// output 128 CTAs; a slab of the inner dimension up to 256 is staged at once, every one of 16
+// warps multiplies its own 16th of it with 4 x 4 outputs per lane (16 FMAs from two 16-byte
+// shared-memory reads), and the 16 partial tiles are added in warp order.  Measured (B200):
+// loss and gradient of a 4-256-256-64 network at batch 256 through host buffers 318 -> 155 us (two thirds of the rest are copies and the fresh host array).
+__global__ void __launch_bounds__(kGemmThreads)
+    GemmKernel(GemmArgs g, GemmArgs h, const float *__restrict__ partials, int count, float scale,
+               float *__restrict__ loss)
+{
+  extern __shared__ __align__(16) float gemm_smem[];
+  __shared__ float red[kGemmWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // Sum over the CTA in a fixed order, valid in thread 0.
+  auto block_sum = [&](float v) {
+    for (int o = 16; o > 0; o >>= 1)
+      v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0)
+      red[warp] = v;
+    __syncthreads();
+    float s = 0.f;
+    if (threadIdx.x == 0)
+      for (int i = 0; i < kGemmWarps; ++i)
+        s += red[i];
+    return s;
+  };
+  int tile = blockIdx.x;
+  if (tile >= g.tiles + h.tiles) {
+    float s = 0.f;
+    for (int i = threadIdx.x; i < count; i += kGemmThreads)
+      s += partials[i];
+    s = block_sum(s);
+    if (threadIdx.x == 0)
+      *loss = s * scale;
     return;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty + 8 * i;
-    if (m >= M)
+  }
+  const bool second = tile >= g.tiles;
+  if (second)
+    tile -= g.tiles;
+  const GemmArgs &p = second ? h : g;
+  const int m0 = tile / p.tiles_n * kTileM, n0 = tile % p.tiles_n * kTileN;
+  float *const As = gemm_smem, *const Bs = gemm_smem + kSlab * kPitchA;
+  const int mm = (lane >> 3) * 4, nn = (lane & 7) * 4;
+  const bool sums = p.row_sum && n0 == 0;
+  float acc[4][4] = {}, sum[4] = {};
+  for (int k0 = 0; k0 < p.K; k0 += kSlab) {
+    if (k0 > 0)
+      __syncthreads();
+    Stage<kTileM, kPitchA>(As, p.A, p.am, p.ak, m0, p.M, k0, p.K);
+    Stage<kTileN, kPitchB>(Bs, p.B, p.bn, p.bk, n0, p.N, k0, p.K);
+    __syncthreads();
+    if (k0 + warp * kWarpK >= p.K)
       continue;
-    const size_t o = static_cast<size_t>(m) * ldc + n;
-    float v = acc[i];
-    if (epilogue == kBiasGelu) {
-      v += bias[n];
-      aux[o] = v;
-      v = Gelu(v);
-    } else if (epilogue == kBias) {
-      v += bias[n];
-    } else if (epilogue == kGeluGrad) {
-      v *= GeluGrad(aux[o]);
+    const float *a = As + warp * kWarpK * kPitchA + mm, *b = Bs + warp * kWarpK * kPitchB + nn;
+#pragma unroll
+    for (int k = 0; k < kWarpK; ++k) {
+      const float4 av = *reinterpret_cast<const float4 *>(a + k * kPitchA);
+      const float4 bv = *reinterpret_cast<const float4 *>(b + k * kPitchB);
+      const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          acc[i][j] = fmaf(ar[i], br[j], acc[i][j]);
+        sum[i] += ar[i];
+      }
     }
-    C[o] = v;
   }
-}
-
-// out[n] = sum over rows m of X[m][n] (fixed row order), for bias gradients.
-__global__ void ColumnSumKernel(int M, int N, const float *__restrict__ X, float *__restrict__ out)
-{
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N)
-    return;
-  float s = 0.f;
-  for (int m = 0; m < M; ++m)
-    s += X[static_cast<size_t>(m) * N + n];
-  out[n] = s;
-}
-
-// d = (y - t) / batch, and per-row partial 0.5 * sum (y - t)^2 for the loss.
-__global__ void OutputDeltaKernel(int batch, int O, const float *__restrict__ y,
-                                  const float *__restrict__ t, float *__restrict__ d,
-                                  float *__restrict__ row_loss)
-{
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= batch)
-    return;
+  // The warps' partial tiles (and row sums) through shared memory.
+  constexpr int kPart = kTileM * kTileN;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4 *>(gemm_smem + warp * kPart + (mm + i) * kTileN + nn) =
+        make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  float *const row = gemm_smem + kGemmWarps * kPart;
+  if (sums && nn == 0)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      row[warp * kTileM + mm + i] = sum[i];
+  __syncthreads();
+  float v = 0.f;
+#pragma unroll
+  for (int w = 0; w < kGemmWarps; ++w)
+    v += gemm_smem[w * kPart + threadIdx.x];
+  if (sums && threadIdx.x < kTileM && m0 + threadIdx.x < p.M) {
+    float s = 0.f;
+    for (int w = 0; w < kGemmWarps; ++w)
+      s += row[w * kTileM + threadIdx.x];
+    p.row_sum[m0 + threadIdx.x] = s;
+  }
+  const int m = m0 + static_cast<int>(threadIdx.x) / kTileN, n = n0 + static_cast<int>(threadIdx.x) % kTileN;
   float l = 0.f;
-  for (int o = 0; o < O; ++o) {
-    const size_t i = static_cast<size_t>(b) * O + o;
-    const float e = y[i] - t[i];
-    d[i] = e / static_cast<float>(batch);
-    l += e * e;
+  if (m < p.M && n < p.N) {
+    const size_t o = static_cast<size_t>(m) * p.ldc + n;
+    if (p.epilogue == kBiasGelu) {
+      v += p.bias[n];
+      p.aux[o] = v;
+      v = Gelu(v);
+    } else if (p.epilogue == kBias) {
+      v += p.bias[n];
+    } else if (p.epilogue == kGeluGrad) {
+      v *= GeluGrad(p.aux[o]);
+    } else if (p.epilogue == kBiasDelta) {
+      v += p.bias[n];
+      const float e = v - p.target[o];
+      p.delta[o] = e / static_cast<float>(p.M);
+      l = 0.5f * e * e;
+    }
+    p.C[o] = v;
   }
-  row_loss[b] = 0.5f * l;
+  if (p.epilogue == kBiasDelta) {
+    l = block_sum(l);
+    if (threadIdx.x == 0)
+      p.loss[tile] = l;
+  }
 }
-
-__global__ void SumKernel(int n, const float *__restrict__ x, float scale, float *__restrict__ out)
-{
-  if (blockIdx.x != 0 || threadIdx.x != 0)
-    return;
-  float s = 0.f;
-  for (int i = 0; i < n; ++i)
-    s += x[i];
-  *out = s * scale;
-}
+static_assert(kTileM * kTileN == kGemmThreads, "one output per thread in the epilogue");
+static_assert(kGemmSmem >= sizeof(float) * kGemmWarps * (kTileM * kTileN + kTileM), "partial tiles fit the staging");
 
 __global__ void GatherRowsKernel(int rows, int width, const int32_t *__restrict__ index,
                                  const float *__restrict__ src, float *__restrict__ dst)
@@ -164,11 +270,20 @@ __global__ void AdamKernel(int64_t n, float *__restrict__ p, const float *__rest
 
 unsigned Grid(size_t threads, int block) { return static_cast<unsigned>((threads + block - 1) / block); }
 
-cudaError_t Gemm(int M, int N, int K, const float *A, int am, int ak, const float *B, int bk, int bn,
-                 float *C, int ldc, int epilogue, const float *bias, float *aux, cudaStream_t st)
+GemmArgs Product(int M, int N, int K, const float *A, int am, int ak, const float *B, int bk, int bn, float *C,
+                 int ldc, int epilogue, const float *bias = nullptr, float *aux = nullptr)
 {
-  const dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-  GemmKernel<<<grid, kThreads, 0, st>>>(M, N, K, A, am, ak, B, bk, bn, C, ldc, epilogue, bias, aux);
+  GemmArgs g{M, N, K, A, am, ak, B, bk, bn, C, ldc, epilogue, bias, aux, nullptr, nullptr, nullptr, nullptr, 0, 0};
+  g.tiles_n = (N + kTileN - 1) / kTileN;
+  g.tiles = g.tiles_n * ((M + kTileM - 1) / kTileM);
+  return g;
+}
+
+// g and optionally h (h.tiles = 0: none); with loss, also the sum of `count` partials.
+cudaError_t Gemm(const GemmArgs &g, const GemmArgs &h, cudaStream_t st, const float *partials = nullptr,
+                 int count = 0, float scale = 0.f, float *loss = nullptr)
+{
+  GemmKernel<<<g.tiles + h.tiles + (loss ? 1 : 0), kGemmThreads, kGemmSmem, st>>>(g, h, partials, count, scale, loss);
   return cudaGetLastError();
 }
 
@@ -178,6 +293,11 @@ Status Mlp::Create(int inputs, int hidden, int outputs, uint64_t seed)
 {
   if (inputs < 1 || hidden < 1 || outputs < 1 || inputs > 4096 || hidden > 4096 || outputs > 4096)
     return Status::kInvalidArgument;
+  if (cudaFuncSetAttribute(GemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return Status::kGpuUnavailable;
+  }
   I_ = inputs;
   H_ = hidden;
   O_ = outputs;
@@ -227,7 +347,8 @@ Status Mlp::EnsureBatch(int batch)
       (s = h2_.ensure(b * H_)) != Status::kOk || (s = a2_.ensure(b * H_)) != Status::kOk ||
       (s = y_.ensure(b * O_)) != Status::kOk || (s = dy_.ensure(b * O_)) != Status::kOk ||
       (s = d2_.ensure(b * H_)) != Status::kOk || (s = d1_.ensure(b * H_)) != Status::kOk ||
-      (s = row_loss_.ensure(b)) != Status::kOk || (s = loss_.ensure(1)) != Status::kOk)
+      (s = row_loss_.ensure(static_cast<size_t>((batch + kTileM - 1) / kTileM) * ((O_ + kTileN - 1) / kTileN))) !=
+          Status::kOk || (s = loss_.ensure(1)) != Status::kOk)
     return s;
   batch_cap_ = batch;
   return Status::kOk;
@@ -246,43 +367,49 @@ Mlp::Views Mlp::Split(float *q) const
   return v;
 }
 
-// y = f(x) for `batch` rows of x (device), keeping pre-activations for Backward.
-Status Mlp::Forward(int batch, const float *x, float *y, cudaStream_t st)
+// y = f(x) for `batch` rows of x (device), keeping pre-activations for Backward; with a
+// target also dy_ and the partials of the loss.
+Status Mlp::Forward(int batch, const float *x, float *y, cudaStream_t st, const float *target)
 {
   const Views w = Split(p_.get());
+  const GemmArgs none{};
   // h1 = GELU(x W1^T + b1): A = x [b][i], B(k=i, n=h) = W1[h][i].
-  if (Gemm(batch, H_, I_, x, I_, 1, w.w1, 1, I_, a1_.get(), H_, kBiasGelu, w.b1, h1_.get(), st) != cudaSuccess ||
-      Gemm(batch, H_, H_, a1_.get(), H_, 1, w.w2, 1, H_, a2_.get(), H_, kBiasGelu, w.b2, h2_.get(), st) != cudaSuccess ||
-      Gemm(batch, O_, H_, a2_.get(), H_, 1, w.w3, 1, H_, y, O_, kBias, w.b3, nullptr, st) != cudaSuccess)
+  GemmArgs out = Product(batch, O_, H_, a2_.get(), H_, 1, w.w3, 1, H_, y, O_, target ? kBiasDelta : kBias, w.b3);
+  out.target = target;
+  out.delta = dy_.get();
+  out.loss = row_loss_.get();
+  if (Gemm(Product(batch, H_, I_, x, I_, 1, w.w1, 1, I_, a1_.get(), H_, kBiasGelu, w.b1, h1_.get()), none, st) !=
+          cudaSuccess ||
+      Gemm(Product(batch, H_, H_, a1_.get(), H_, 1, w.w2, 1, H_, a2_.get(), H_, kBiasGelu, w.b2, h2_.get()), none,
+           st) != cudaSuccess ||
+      Gemm(out, none, st) != cudaSuccess)
     return Status::kInternalError;
+  loss_partials_ = out.tiles;
   launches_ += 3;
   return Status::kOk;
 }
 
-// Gradient of 0.5 / batch * sum (y - t)^2 into g_, after Forward(x) -> y_.
-Status Mlp::Backward(int batch, const float *x, const float *t, cudaStream_t st)
+// Gradient of 0.5 / batch * sum (y - t)^2 into g_ and the loss into loss_, after
+// Forward(x, y_, t).
+Status Mlp::Backward(int batch, const float *x, cudaStream_t st)
 {
   const Views w = Split(p_.get());
   const Views g = Split(g_.get());
-  OutputDeltaKernel<<<Grid(batch, 128), 128, 0, st>>>(batch, O_, y_.get(), t, dy_.get(), row_loss_.get());
-  // dW3 = dy^T a2 (O x H), db3 = colsum(dy); d2 = (dy W3) * GELU'(h2).
-  if (cudaGetLastError() != cudaSuccess ||
-      Gemm(O_, H_, batch, dy_.get(), 1, O_, a2_.get(), H_, 1, g.w3, H_, kStore, nullptr, nullptr, st) != cudaSuccess)
+  // dW3 = dy^T a2 (O x H), db3 = colsum(dy) | d2 = (dy W3) * GELU'(h2); dW2 = d2^T a1, db2 |
+  // d1 = (d2 W2) * GELU'(h1); dW1 = d1^T x, db1 | the loss.
+  GemmArgs w3 = Product(O_, H_, batch, dy_.get(), 1, O_, a2_.get(), H_, 1, g.w3, H_, kStore);
+  GemmArgs w2 = Product(H_, H_, batch, d2_.get(), 1, H_, a1_.get(), H_, 1, g.w2, H_, kStore);
+  GemmArgs w1 = Product(H_, I_, batch, d1_.get(), 1, H_, x, I_, 1, g.w1, I_, kStore);
+  w3.row_sum = g.b3;
+  w2.row_sum = g.b2;
+  w1.row_sum = g.b1;
+  if (Gemm(Product(batch, H_, O_, dy_.get(), O_, 1, w.w3, H_, 1, d2_.get(), H_, kGeluGrad, nullptr, h2_.get()), w3,
+           st) != cudaSuccess ||
+      Gemm(Product(batch, H_, H_, d2_.get(), H_, 1, w.w2, H_, 1, d1_.get(), H_, kGeluGrad, nullptr, h1_.get()), w2,
+           st) != cudaSuccess ||
+      Gemm(w1, GemmArgs{}, st, row_loss_.get(), loss_partials_, 1.0f / batch, loss_.get()) != cudaSuccess)
     return Status::kInternalError;
-  ColumnSumKernel<<<Grid(O_, 128), 128, 0, st>>>(batch, O_, dy_.get(), g.b3);
-  if (cudaGetLastError() != cudaSuccess ||
-      Gemm(batch, H_, O_, dy_.get(), O_, 1, w.w3, H_, 1, d2_.get(), H_, kGeluGrad, nullptr, h2_.get(), st) != cudaSuccess ||
-      Gemm(H_, H_, batch, d2_.get(), 1, H_, a1_.get(), H_, 1, g.w2, H_, kStore, nullptr, nullptr, st) != cudaSuccess)
-    return Status::kInternalError;
-  ColumnSumKernel<<<Grid(H_, 128), 128, 0, st>>>(batch, H_, d2_.get(), g.b2);
-  if (cudaGetLastError() != cudaSuccess ||
-      Gemm(batch, H_, H_, d2_.get(), H_, 1, w.w2, H_, 1, d1_.get(), H_, kGeluGrad, nullptr, h1_.get(), st) != cudaSuccess ||
-      Gemm(H_, I_, batch, d1_.get(), 1, H_, x, I_, 1, g.w1, I_, kStore, nullptr, nullptr, st) != cudaSuccess)
-    return Status::kInternalError;
-  ColumnSumKernel<<<Grid(H_, 128), 128, 0, st>>>(batch, H_, d1_.get(), g.b1);
-  if (cudaGetLastError() != cudaSuccess)
-    return Status::kInternalError;
-  launches_ += 9;
+  launches_ += 3;
   return Status::kOk;
 }
 
@@ -315,17 +442,19 @@ Status Mlp::LossGradient(int batch, const float *x_host, const float *t_host, fl
   Status s = EnsureBatch(batch);
   if (s != Status::kOk || (s = x_.upload(x_host, static_cast<size_t>(batch) * I_)) != Status::kOk ||
       (s = t_.upload(t_host, static_cast<size_t>(batch) * O_)) != Status::kOk ||
-      (s = Forward(batch, x_.get(), y_.get(), nullptr)) != Status::kOk ||
-      (s = Backward(batch, x_.get(), t_.get(), nullptr)) != Status::kOk)
+      (s = Forward(batch, x_.get(), y_.get(), nullptr, t_.get())) != Status::kOk ||
+      (s = Backward(batch, x_.get(), nullptr)) != Status::kOk)
     return s;
-  SumKernel<<<1, 1>>>(batch, row_loss_.get(), 1.0f / batch, loss_.get());
-  if (cudaGetLastError() != cudaSuccess)
+  // The loss into pinned memory, so that the gradient's copy is the only wait.
+  if (loss && ((s = host_loss_.ensure(1)) != Status::kOk ||
+               cudaMemcpyAsync(host_loss_.get(), loss_.get(), sizeof(float), cudaMemcpyDeviceToHost, nullptr) !=
+                   cudaSuccess))
+    return s != Status::kOk ? s : Status::kInternalError;
+  if ((gradient_host ? cudaMemcpy(gradient_host, g_.get(), sizeof(float) * ParameterCount(), cudaMemcpyDeviceToHost)
+                     : cudaStreamSynchronize(nullptr)) != cudaSuccess)
     return Status::kInternalError;
-  if (loss && cudaMemcpy(loss, loss_.get(), sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
-    return Status::kInternalError;
-  if (gradient_host && cudaMemcpy(gradient_host, g_.get(), sizeof(float) * ParameterCount(),
-                                  cudaMemcpyDeviceToHost) != cudaSuccess)
-    return Status::kInternalError;
+  if (loss)
+    *loss = *host_loss_.get();
   return Status::kOk;
 }
 
@@ -358,8 +487,8 @@ Status Mlp::Train(int samples, const float *x_host, const float *t_host, int epo
       GatherRowsKernel<<<Grid(static_cast<size_t>(batch) * O_, kThreads), kThreads>>>(
           batch, O_, perm.get() + first, ts.get(), t_.get());
       if (cudaGetLastError() != cudaSuccess ||
-          (s = Forward(batch, x_.get(), y_.get(), nullptr)) != Status::kOk ||
-          (s = Backward(batch, x_.get(), t_.get(), nullptr)) != Status::kOk)
+          (s = Forward(batch, x_.get(), y_.get(), nullptr, t_.get())) != Status::kOk ||
+          (s = Backward(batch, x_.get(), nullptr)) != Status::kOk)
         return s != Status::kOk ? s : Status::kInternalError;
       ++steps_;
       const double c1 = 1.0 - std::pow(double(kBeta1), double(steps_));
@@ -373,11 +502,10 @@ Status Mlp::Train(int samples, const float *x_host, const float *t_host, int epo
     }
   }
   // Loss over the whole training set with the final parameters.
-  if ((s = Forward(samples, xs.get(), y_.get(), nullptr)) != Status::kOk ||
-      (s = Backward(samples, xs.get(), ts.get(), nullptr)) != Status::kOk)
+  if ((s = Forward(samples, xs.get(), y_.get(), nullptr, ts.get())) != Status::kOk ||
+      (s = Backward(samples, xs.get(), nullptr)) != Status::kOk)
     return s;
-  SumKernel<<<1, 1>>>(samples, row_loss_.get(), 1.0f / samples, loss_.get());
-  if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+  if (cudaDeviceSynchronize() != cudaSuccess)
     return Status::kInternalError;
   if (final_loss && cudaMemcpy(final_loss, loss_.get(), sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
     return Status::kInternalError;

@@ -38,14 +38,15 @@ private:
   };
   Views Split(float *q) const;
   Status EnsureBatch(int batch);
-  Status Forward(int batch, const float *x, float *y, cudaStream_t st);
-  Status Backward(int batch, const float *x, const float *t, cudaStream_t st);
+  Status Forward(int batch, const float *x, float *y, cudaStream_t st, const float *target = nullptr);
+  Status Backward(int batch, const float *x, cudaStream_t st);
 
   int I_ = 0, H_ = 0, O_ = 0;
-  int batch_cap_ = 0;
+  int batch_cap_ = 0, loss_partials_ = 0;
   int64_t steps_ = 0, launches_ = 0;
   DeviceArray<float> p_, g_, m_, v_;
-  DeviceArray<float> x_, t_, h1_, a1_, h2_, a2_, y_, dy_, d2_, d1_, row_loss_, loss_;
+  DeviceArray<float> x_, t_, h1_, a1_, h2_, a2_, y_, dy_, d2_, d1_, row_loss_ /* tile by tile */, loss_;
+  PinnedArray<float> host_loss_;
 };
 
 } // namespace fg
