@@ -749,10 +749,19 @@ int fg_postprocess_compute_device(fg_postprocess *pp, int32_t items, const doubl
       return ToInt(s);
     }
   }
-  const int ctas = fg::PostprocessCtas(E, items);
-  const size_t partial_count = static_cast<size_t>(ctas) * items * 3;
-  const size_t total = partial_count + P * items;
-  if ((s = pp->out.ensure(total)) != Status::kOk || (s = pp->host_out.ensure(total)) != Status::kOk)
+  const size_t groups = static_cast<size_t>(fg::PostprocessGroups(items));
+  if (pp->arrived.capacity() < groups) {
+    if ((s = pp->arrived.ensure(groups)) != Status::kOk)
+      return ToInt(s);
+    if (cudaMemsetAsync(pp->arrived.get(), 0, groups * sizeof(unsigned), stream) != cudaSuccess) {
+      cudaGetLastError();
+      pp->arrived.reset();
+      return ToInt(Status::kInternalError);
+    }
+  }
+  const size_t sums = 3 * static_cast<size_t>(items);
+  if ((s = pp->out.ensure(fg::PostprocessPartials(E, items))) != Status::kOk ||
+      (s = pp->host_out.ensure(sums + P * items)) != Status::kOk)
     return ToInt(s);
   fg::PostprocessDevice d{};
   const double *g = pp->geometry.get();
@@ -772,17 +781,16 @@ int fg_postprocess_compute_device(fg_postprocess *pp, int32_t items, const doubl
   d.E = E;
   d.N = N;
   d.items = items;
-  d.ctas = ctas;
+  d.ctas = fg::PostprocessCtas(E, items);
   d.probes = Pn;
   d.a = a;
   d.b1 = b1;
   d.b2 = b2;
   d.partials = pp->out.get();
-  d.radial = d.partials + partial_count;
-  if (fg::LaunchPostprocess(d, stream) != cudaSuccess ||
-      cudaMemcpyAsync(pp->host_out.get(), pp->out.get(), total * sizeof(double), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess) {
+  d.arrived = pp->arrived.get();
+  d.sums = pp->host_out.get();
+  d.radial = d.sums + sums;
+  if (fg::LaunchPostprocess(d, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess) {
     cudaGetLastError();
     return ToInt(Status::kInternalError);
   }
@@ -790,18 +798,15 @@ int fg_postprocess_compute_device(fg_postprocess *pp, int32_t items, const doubl
   for (int32_t i = 0; i < items; ++i) {
     fg_postprocess_result &r = results[i];
     r = fg_postprocess_result{};
-    for (int c = 0; c < ctas; ++c) {
-      const double *q = h + (static_cast<size_t>(c) * items + i) * 3;
-      r.force_x_n += q[0];
-      r.force_y_n += q[1];
-      r.torque_nm += q[2];
-    }
-    if (P)
-      std::copy(h + partial_count + P * i, h + partial_count + P * (i + 1), radial + P * i);
+    r.force_x_n = h[3 * i];
+    r.force_y_n = h[3 * i + 1];
+    r.torque_nm = h[3 * i + 2];
     r.status = ToInt(std::isfinite(r.force_x_n) && std::isfinite(r.force_y_n) && std::isfinite(r.torque_nm)
                          ? Status::kOk
                          : Status::kNumericalNonfinite);
   }
+  if (P)
+    std::copy(h + sums, h + sums + P * items, radial);
   return ToInt(Status::kOk);
 }
 

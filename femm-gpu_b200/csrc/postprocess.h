@@ -65,8 +65,8 @@ Status ComputeTangentPostprocess(const HostModel &model, const PostprocessPlan &
                                  const double *base_b2, const double *da, const double *db1,
                                  const double *db2, fg_postprocess_result *result, double *radial_b);
 
-// Device form: force / torque partial sums per (CTA, item) and the air-gap samples of every
-// (item, probe) from the corner recipes, in one launch.
+// Device form: force / torque of every item and the air-gap samples of every (item, probe)
+// from the corner recipes, in one launch.
 struct PostprocessDevice {
   const double *hx, *hy, *weight, *cx, *cy; // [E]
   const CornerStencil *corners;             // [3 * probes]
@@ -75,9 +75,13 @@ struct PostprocessDevice {
   const double *probe;                      // [probes][5]: lambda 0..2, cos, sin
   int32_t E, N, items, ctas, probes;
   const double *a, *b1, *b2; // item-major solutions
-  double *partials;          // [ctas][items][3]
-  double *radial;            // [items][probes]
+  double *partials;          // PostprocessPartials(E, items)
+  unsigned *arrived;         // [item groups], zero between launches
+  double *sums;              // [items][3]: force x, y, torque (pinned host memory)
+  double *radial;            // [items][probes] (pinned host memory)
 };
+int PostprocessGroups(int32_t items);
+size_t PostprocessPartials(int32_t E, int32_t items);
 int PostprocessCtas(int32_t E, int32_t items);
 cudaError_t LaunchPostprocess(const PostprocessDevice &p, cudaStream_t stream);
 
@@ -90,6 +94,7 @@ struct fg_postprocess {
   fg::DeviceArray<double> geometry; // hx, hy, weight, cx, cy [5][E]; probes [5P]; terms w, tx, ty, len
   fg::DeviceArray<int32_t> terms;   // term_elem, term_node
   fg::DeviceArray<fg::CornerStencil> corners;
-  fg::DeviceArray<double> out;      // partials, radial
-  fg::PinnedArray<double> host_out;
+  fg::DeviceArray<double> out;      // partials
+  fg::DeviceArray<unsigned> arrived;
+  fg::PinnedArray<double> host_out; // sums, radial: written by the kernel
 };

@@ -562,6 +562,10 @@ class FgPostprocessResult(C.Structure):
                 ("force_y_n", C.c_double), ("torque_nm", C.c_double)]
 
 
+_POST_DTYPE = np.dtype([("status", np.int32), ("reserved", np.int32), ("force", np.float64, 2),
+                        ("torque", np.float64)])
+
+
 @dataclass
 class PostprocessResult:
     status: np.ndarray       # [items]
@@ -618,12 +622,11 @@ class Postprocess:
             raise FgError(st, "fg_postprocess_mask")
         return out
 
-    def _result(self, res, radial):
-        k = len(res)
-        return PostprocessResult(
-            status=np.array([res[i].status for i in range(k)]),
-            force=np.array([[res[i].force_x_n, res[i].force_y_n] for i in range(k)]).reshape(k, 2),
-            torque=np.array([res[i].torque_nm for i in range(k)]), radial_b=radial)
+    def _result(self, res, radial, count):
+        # The C array as one structured view instead of an attribute at a time.
+        r = np.frombuffer(res, dtype=_POST_DTYPE, count=count)
+        return PostprocessResult(status=r["status"].astype(np.int64), force=r["force"].copy(),
+                                 torque=r["torque"].copy(), radial_b=radial)
 
     def compute(self, a, b1, b2) -> PostprocessResult:
         """Host solutions: a [k, N], b1 / b2 [k, E]."""
@@ -637,7 +640,7 @@ class Postprocess:
                                           _p(radial) if self.probes else None)
         if st:
             raise FgError(st, "fg_postprocess_compute")
-        return self._result([res[i] for i in range(k)], radial)
+        return self._result(res, radial, k)
 
     def tangent(self, base_b1, base_b2, da, db1, db2) -> PostprocessResult:
         """Derivatives about base B of tangent solutions da [m, N], db1 / db2 [m, E]."""
@@ -653,7 +656,7 @@ class Postprocess:
                                           _p(radial) if self.probes else None)
         if st:
             raise FgError(st, "fg_postprocess_tangent")
-        return self._result([res[i] for i in range(m)], radial)
+        return self._result(res, radial, m)
 
     def compute_device(self, k, a_ptr, b1_ptr, b2_ptr, stream=0) -> PostprocessResult:
         """Device solutions (item-major) by pointer, e.g. torch tensors' data_ptr()."""
@@ -664,4 +667,4 @@ class Postprocess:
             _p(radial) if self.probes else None, C.c_void_p(stream))
         if st:
             raise FgError(st, "fg_postprocess_compute_device")
-        return self._result([res[i] for i in range(k)], radial)
+        return self._result(res, radial, k)
