@@ -104,6 +104,11 @@ struct PcgArgs {
   // shared memory (needs host_slice_off), 2 off.  The same bits either way.  row_groups and
   // resident_offset are set by LaunchPcg.
   int32_t resident_request, row_groups, resident_offset;
+  // Window form (FP64 Jacobi; pcg_window.cuh): window_request 1 asks for it where the resident
+  // form does not fit and this one does (the same bits again); bandwidth: the operator's
+  // largest |row - column|, 0 where the caller does not know it; window_rows is set by
+  // LaunchPcg.
+  int32_t window_request, bandwidth, window_rows;
   // One-reduction form (FP64 Jacobi only; pcg1r_kernel.cuh): t0 / t1 are two more
   // vectors of [n_pad][kp] doubles, and partials must hold 2 x 96 x grid doubles.
   int32_t one_reduction;
@@ -140,6 +145,8 @@ cudaError_t LaunchBlockInverse(const DevicePlan &p, int kp, int items, int bs, c
                                float *out32, int32_t *fallbacks, cudaStream_t stream);
 // Whether LaunchPcg would run args in the resident form.
 bool PcgResident(const PcgArgs &args);
+// Whether the window form could run them.
+bool PcgWindow(const PcgArgs &args);
 // Cooperative persistent PCG; *grid_out receives the number of CTAs used.
 cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t stream);
 int PcgMaxGrid(int kp);

@@ -25,6 +25,8 @@ const void *PcgKernelF64Resident(int kp, bool shared, int *entry);
 // values read from L2 (always with one); *step receives the bytes of a warp-step besides its
 // entries.
 const void *PcgKernelF64ResidentSteps(int kp, bool shared, bool stream, int groups, int *step, int *entry);
+// The window form; q_global: q in global memory.
+const void *PcgKernelF64Window(int kp, bool q_global);
 
 namespace
 {
@@ -230,7 +232,48 @@ bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
   return false;
 }
 
+// The window form's launch, if the window (all rows that the operator's bandwidth can reach from
+// a round's tile, and the tiles of the rounds in flight) fits in shared memory, with q beside it
+// if that fits too.  `out` receives kernel, CTAs and shared memory; returns the window's rows,
+// 0 if none.  Not where a CTA's two neighbourhoods have more rows than twice its own: filling
+// the window would be most of the work.  (Who asks for the form has timed it: a plan's tuner.)
+int ChooseWindow(const PcgArgs &args, int groups, ResidentShape *out)
+{
+  if (args.resident_request == 2 || args.precision != 0 || args.blocks || args.one_reduction || args.reliable ||
+      args.bandwidth <= 0 || !args.host_slice_off || !args.value_item || !args.diag_item)
+    return 0;
+  const int s = 32 * ItemsPerThread(args.kp, 0) / args.kp, tile = kPcgWarps * s;
+  const long long ws = args.n_pad / s, ctas = (groups + 1) / 2;
+  const long long rows = 2ll * args.bandwidth + 4 * tile;
+  if (ws < groups || 2ll * args.bandwidth > 2 * (ws / ctas) * s)
+    return 0;
+  long long most = 0;
+  for (int c = 0; c < ctas; ++c) {
+    const long long w0 = ws * (2 * c) / groups, w1 = ws * std::min(groups, 2 * c + 2) / groups;
+    most = std::max(most, w1 - w0);
+  }
+  const long long ring = rows * args.kp * 8, q = most * s * args.kp * 8;
+  for (const bool q_global : {false, true}) {
+    const void *kernel = PcgKernelF64Window(args.kp, q_global);
+    const long long total = ring + (q_global ? 0 : q);
+    if (!kernel || total > 227 * 1024 || KernelGrid(kernel, static_cast<size_t>(total), kPcgThreads, 1) < ctas)
+      continue;
+    *out = ResidentShape{kernel, static_cast<int>(ctas), 0, static_cast<size_t>(total)};
+    return static_cast<int>(rows);
+  }
+  return 0;
+}
+
 } // namespace
+
+bool PcgWindow(const PcgArgs &args)
+{
+  ResidentShape shape;
+  const int max_grid = PcgMaxGrid(args.kp);
+  const bool fits = max_grid > 0 && ChooseWindow(args, RowGroups(args, max_grid), &shape) > 0;
+  cudaGetLastError(); // a size beyond the shared-memory limit is not an error here
+  return fits;
+}
 
 bool PcgResident(const PcgArgs &args)
 {
@@ -262,7 +305,12 @@ cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t 
   const int warp_slices = args.n_pad / rows_per_warp;
   const int grid = RowGroups(args, max_grid);
   ResidentShape resident;
-  if (ChooseResident(args, grid, &resident)) {
+  bool on_chip = ChooseResident(args, grid, &resident);
+  if (!on_chip && args.window_request == 1) {
+    args.window_rows = ChooseWindow(args, grid, &resident);
+    on_chip = args.window_rows > 0;
+  }
+  if (on_chip) {
     args.row_groups = grid;
     args.resident_offset = resident.offset;
     cudaError_t e = cudaMemsetAsync(args.barrier, 0, sizeof(unsigned), stream);

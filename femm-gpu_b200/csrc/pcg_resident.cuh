@@ -238,8 +238,9 @@ __device__ __forceinline__ void SendPartials(int rank, const Mailboxes<KP> &mail
 }
 
 // ... then it sums the items this CTA owns and sends their results to every CTA (or sums
-// every item itself, direct).  Lane `item` leaves with the item's sums.
-template <int KP, int GV, int Q>
+// every item itself, direct).  Lane `item` leaves with the item's sums.  kFence: and with
+// everything acquired that the CTAs had released with their partials.  N: partials a lane polls at once.
+template <int KP, int GV, int Q, bool kFence = false, int N = 5>
 __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailboxes<KP> &mail,
                                         ResidentShared<KP, GV> &sm, int r, double (&sum)[Q])
 {
@@ -283,7 +284,6 @@ __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailbo
 #pragma unroll
     for (int q = 0; q < Q; ++q)
       s[q] = 0.0;
-    constexpr int N = 5;
     for (int g0 = 0; g0 < G; g0 += 32 * N) {
       double y[N][Q];
       const int count = (G - g0 - lane + 31) >> 5;
@@ -302,6 +302,8 @@ __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailbo
       for (int q = 0; q < Q; ++q)
         s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
     const double m[2] = {Sendable(s[0]), Sendable(s[Q - 1])};
+    if constexpr (kFence)
+      FenceAcqRel();
     for (int c = lane; c < mail.ctas; c += 32)
       StoreMessage<2>(mail.Result(r, c, it), m);
   }
@@ -310,6 +312,8 @@ __device__ __forceinline__ void Collect(const PcgArgs &a, int rank, const Mailbo
   __syncwarp();
   sum[Q - 1] = y[0][1];
   sum[0] = y[0][0];
+  if constexpr (kFence)
+    FenceAcqRel();
 }
 
 // The same sums in the rare phases (set-up, verification, the end of the budget), behind a

@@ -177,6 +177,10 @@ Status Plan::Upload()
   FG_UP(row_len_, h.row_len);
   FG_UP(slice_off_, h.slice_off);
   FG_UP(sell_col_, h.sell_col);
+  bandwidth_ = 0;
+  for (int32_t r = 0; r < h.n; ++r)
+    for (int32_t e = h.row_offsets[r]; e < h.row_offsets[r + 1]; ++e)
+      bandwidth_ = std::max(bandwidth_, std::abs(h.columns[e] - r));
   FG_UP(contrib_off_, h.contrib_off);
   FG_UP(contrib_, h.contrib);
   FG_UP(rhs_off_, h.rhs_off);
@@ -346,6 +350,7 @@ Status Plan::RunPcg(int kp, int items, uint32_t mask, double tolerance, int max_
   a.items = items;
   a.slice_off = slice_off_.get();
   a.host_slice_off = host_.slice_off.data();
+  a.bandwidth = bandwidth_;
   a.row_len = row_len_.get();
   a.sell_col = sell_col_.get();
   a.values = values_.get();
@@ -417,9 +422,9 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     sh.block_size = a.blocks ? a.block_size : 0;
     // Candidates: 512-thread CTAs with the ring on / off (only 16-byte item vectors of
     // per-item operators can use it) x column cache off / on, and 1024-thread CTAs with the
-    // ring (FP64 Jacobi, where the launch admits them).  Each runs kTuneIterations CG
-    // iterations of this very system (tolerance 0: no item stops early); the real launch
-    // follows and overwrites every vector the timing runs wrote.
+    // ring (FP64 Jacobi, where the launch admits them); beside them the window form, where it
+    // fits.  Each runs kTuneIterations CG iterations of this very system (tolerance 0: no item
+    // stops early); the real launch follows and overwrites every vector the timing runs wrote.
     const int iv = a.precision == 0 ? (a.kp >= 2 ? 2 : 1) : (a.kp >= 4 ? 4 : (a.kp >= 2 ? 2 : 1));
     const bool ring_possible = (a.precision == 0 ? 8 : 4) * iv == 16 && a.value_item;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -434,6 +439,8 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     const bool resident = PcgResident(a);
     const int iterations = resident ? kTuneIterationsResident : kTuneIterations;
     const int rounds = resident ? 1 : kTuneRounds;
+    const bool window = !resident && PcgWindow(a);
+    double window_us = 0.0;
     PcgArgs t = a;
     t.tolerance = 0.0;
     t.item_tolerance = nullptr;
@@ -446,10 +453,12 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     else
       timing_.kernel_launches += 1;
     for (int round = 0; round < rounds; ++round)
-      for (int c = 0; c < 5; ++c) {
+      for (int c = 0; c < 6; ++c) {
         const int ring = c % 2 == 0 ? 1 : 2, cache = c == 2 || c == 3 ? 1 : 2;
-        if (ring == 1 && !ring_possible)
+        if (c < 5 ? ring == 1 && !ring_possible : !window)
           continue;
+        t.resident_request = c < 5 ? 2 : 0;
+        t.window_request = c < 5 ? 0 : 1;
         t.ring_request = ring;
         t.col_cache_request = cache;
         t.block_request = c == 4 ? 1 : 2;
@@ -465,7 +474,9 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         if (c == 4 && threads != 1024)
           continue; // the launch fell back to 512 threads: not a candidate of its own
         const double us = 1e3 * ms / iterations;
-        if (sh.us_per_iteration[c] == 0.0) {
+        if (c == 5)
+          window_us = window_us == 0.0 ? us : std::min(window_us, us);
+        else if (sh.us_per_iteration[c] == 0.0) {
           ++sh.candidates;
           sh.us_per_iteration[c] = us;
         } else if (us < sh.us_per_iteration[c]) {
@@ -480,7 +491,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         sh.column_cache = c == 2 || c == 3 ? 1 : 0;
         sh.threads_per_block = c == 4 ? 1024 : 512;
       }
-    sh.resident = resident ? 1 : 0;
+    sh.resident = resident ? 1 : (window_us > 0.0 && window_us < best ? 2 : 0);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (sh.candidates > 0)
@@ -492,6 +503,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     a.block_request = it->second.threads_per_block == 1024 ? 1 : 2;
     if (!it->second.resident)
       a.resident_request = 2;
+    a.window_request = it->second.resident == 2 ? 1 : 0;
   }
   return LaunchPcg(a, grid, block, stream);
 }

@@ -441,7 +441,8 @@ class Plan:
         return [{"items": a.items, "precision": a.precision, "block_size": a.block_size,
                  "value_ring": bool(a.value_ring), "column_cache": bool(a.column_cache),
                  "candidates": a.candidates, "us_per_iteration": list(a.us_per_iteration),
-                 "threads_per_block": a.threads_per_block, "resident": bool(a.resident)}
+                 "threads_per_block": a.threads_per_block, "resident": a.resident == 1,
+                 "window": a.resident == 2}
                 for a in arr[:n]]
 
 

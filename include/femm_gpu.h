@@ -364,7 +364,7 @@ typedef struct fg_pcg_shape {
    * cache off; 0 if not timed */
   double us_per_iteration[5];
   int32_t threads_per_block; /* the fastest of these: 512 or 1024 (the same bits either way) */
-  int32_t resident;          /* 1: the resident form (not among these) was faster and is used */
+  int32_t resident;          /* not among these and used instead: 1 the resident form, 2 the window form */
 } fg_pcg_shape;
 int fg_plan_pcg_shapes(const fg_plan *plan, int32_t capacity, fg_pcg_shape *shapes);
 
