@@ -205,13 +205,13 @@ bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
       w += n;
     }
   }
-  auto fits = [&](const void *kernel, long long step_bytes, long long entry_bytes) {
+  auto fits = [&](const void *kernel, long long step_bytes, long long entry_bytes, bool stream) {
     long long data = 0, most = 0;
     for (int c = 0; c < ctas; ++c) {
       data = std::max(data, steps[c] * step_bytes + entries[c] * entry_bytes);
       most = std::max(most, steps[c]);
     }
-    const long long total = data + (most + 1) * 4;
+    const long long total = data + (most + 1 + (stream ? most : 0)) * 4;
     if (!kernel || total > 227 * 1024 || KernelGrid(kernel, static_cast<size_t>(total), kPcgThreads, 1) < ctas)
       return false;
     *out = ResidentShape{kernel, ctas, static_cast<int>(data), static_cast<size_t>(total)};
@@ -219,14 +219,14 @@ bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
   };
   if (per_cta == 1 && ws <= static_cast<long long>(groups) * kPcgWarps) {
     const void *kernel = PcgKernelF64Resident(args.kp, shared, &entry);
-    if (fits(kernel, 0, entry))
+    if (fits(kernel, 0, entry, false))
       return true;
   }
   for (const bool stream : {false, true}) {
     if (!stream && per_cta == 1)
       continue;
     const void *kernel = PcgKernelF64ResidentSteps(args.kp, shared, stream, per_cta, &step, &entry);
-    if (fits(kernel, step, entry))
+    if (fits(kernel, step, entry, stream))
       return true;
   }
   return false;
