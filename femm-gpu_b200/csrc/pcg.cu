@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace fg
@@ -60,6 +61,38 @@ size_t StagingBytes(int kp, int precision, int bs)
   return static_cast<size_t>(kPcgWarps) * u * kp * (precision == 0 ? 8 : 4);
 }
 
+// The most dynamic shared memory a launch of `kernel` may ask for on `device`: what a CTA may
+// opt in to, less the kernel's static part; 0 on failure.  The attribute that admits it belongs
+// to the kernel, which every plan and thread of the process launches, so it is set once, to
+// this limit: set to a launch's own size it could be lowered by another thread's smaller launch
+// before this one's.
+size_t DynamicLimit(const void *kernel, int device)
+{
+  struct Known {
+    const void *kernel;
+    int device;
+    size_t limit;
+  };
+  static Known known[512]; // more than there are kernels, for several devices; then it is set again
+  static int count = 0;
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
+  for (int i = 0; i < count; ++i)
+    if (known[i].kernel == kernel && known[i].device == device)
+      return known[i].limit;
+  cudaFuncAttributes attr;
+  int most = 0;
+  if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
+      cudaFuncGetAttributes(&attr, kernel) != cudaSuccess || attr.sharedSizeBytes >= static_cast<size_t>(most))
+    return 0;
+  const size_t limit = static_cast<size_t>(most) - attr.sharedSizeBytes;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)) != cudaSuccess)
+    return 0;
+  if (count < static_cast<int>(sizeof(known) / sizeof(known[0])))
+    known[count++] = Known{kernel, device, limit};
+  return limit;
+}
+
 // Co-resident CTAs of one kernel shape (at most `cap` per SM), 0 on failure.
 int KernelGrid(const void *kernel, size_t smem, int threads = kPcgThreads, int cap = 2)
 {
@@ -67,9 +100,7 @@ int KernelGrid(const void *kernel, size_t smem, int threads = kPcgThreads, int c
   if (!kernel || cudaGetDevice(&device) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
     return 0;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
+  if (smem > 0 && smem > DynamicLimit(kernel, device))
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
     return 0;
