@@ -7,7 +7,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 namespace fg
 {
@@ -224,41 +223,46 @@ bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
   if (!PcgKernelF64ResidentSteps(args.kp, shared, true, per_cta, &step, &entry) ||
       (ws / ctas) * (step + entry) > 227 * 1024)
     return false;
-  // Steps and operator entries of every CTA.
-  std::vector<long long> steps(ctas), entries(ctas);
-  for (int c = 0; c < ctas; ++c) {
-    const long long w0 = ws * (c * per_cta) / groups, w1 = ws * std::min(groups, (c + 1) * per_cta) / groups;
-    steps[c] = w1 - w0;
-    for (long long w = w0; w < w1;) { // whole slices at a time
-      const long long slice = (w * s) >> 5, end = ((slice + 1) * 32) / s;
-      const long long n = (end < w1 ? end : w1) - w;
-      entries[c] += n * ((args.host_slice_off[slice + 1] - args.host_slice_off[slice]) / 32);
-      w += n;
-    }
-  }
-  auto fits = [&](const void *kernel, long long step_bytes, long long entry_bytes, bool stream) {
-    long long data = 0, most = 0;
-    for (int c = 0; c < ctas; ++c) {
-      data = std::max(data, steps[c] * step_bytes + entries[c] * entry_bytes);
-      most = std::max(most, steps[c]);
-    }
-    const long long total = data + (most + 1 + (stream ? most : 0)) * 4;
-    if (!kernel || total > 227 * 1024 || KernelGrid(kernel, static_cast<size_t>(total), kPcgThreads, 1) < ctas)
-      return false;
-    *out = ResidentShape{kernel, ctas, static_cast<int>(data), static_cast<size_t>(total)};
-    return true;
-  };
+  // The forms to try, in order, and the bytes of the largest share of a CTA in each.  (No heap:
+  // fg_csr_pcg_noalloc comes here, and nothing may throw.)
+  struct Form {
+    const void *kernel;
+    bool stream;
+    long long step, entry, data;
+  } forms[3];
+  int count = 0;
   if (per_cta == 1 && ws <= static_cast<long long>(groups) * kPcgWarps) {
     const void *kernel = PcgKernelF64Resident(args.kp, shared, &entry);
-    if (fits(kernel, 0, entry, false))
-      return true;
+    forms[count++] = Form{kernel, false, 0, entry, 0};
   }
   for (const bool stream : {false, true}) {
     if (!stream && per_cta == 1)
       continue;
     const void *kernel = PcgKernelF64ResidentSteps(args.kp, shared, stream, per_cta, &step, &entry);
-    if (fits(kernel, step, entry, stream))
-      return true;
+    forms[count++] = Form{kernel, stream, step, entry, 0};
+  }
+  long long most = 0; // steps of a CTA
+  for (int c = 0; c < ctas; ++c) {
+    const long long w0 = ws * (c * per_cta) / groups, w1 = ws * std::min(groups, (c + 1) * per_cta) / groups;
+    long long entries = 0;
+    for (long long w = w0; w < w1;) { // whole slices at a time
+      const long long slice = (w * s) >> 5, end = ((slice + 1) * 32) / s;
+      const long long n = (end < w1 ? end : w1) - w;
+      entries += n * ((args.host_slice_off[slice + 1] - args.host_slice_off[slice]) / 32);
+      w += n;
+    }
+    most = std::max(most, w1 - w0);
+    for (int f = 0; f < count; ++f)
+      forms[f].data = std::max(forms[f].data, (w1 - w0) * forms[f].step + entries * forms[f].entry);
+  }
+  for (int f = 0; f < count; ++f) {
+    const Form &form = forms[f];
+    const long long total = form.data + (most + 1 + (form.stream ? most : 0)) * 4;
+    if (!form.kernel || total > 227 * 1024 ||
+        KernelGrid(form.kernel, static_cast<size_t>(total), kPcgThreads, 1) < ctas)
+      continue;
+    *out = ResidentShape{form.kernel, ctas, static_cast<int>(form.data), static_cast<size_t>(total)};
+    return true;
   }
   return false;
 }
