@@ -23,14 +23,16 @@
 // with cudaGetSymbolAddress and caches it; make that first call before any stream
 // capture begins.
 //
-// Host waits: every call synchronises `stream` -- once after the set-up kernel, to read
-// what it found wrong with the system, and again after the solve, to read its status before
-// x is written -- so it returns only when x and info are final.
+// Host waits: every call synchronises `stream` three times -- after the set-up kernel, to read
+// what it found wrong with the system and where its slices start; after the solve, to read its
+// status before x is written; and after the copy of x -- so it returns only when x and info are
+// final.
 #include "femm_gpu.h"
 #include "common.h"
 #include "kernels.cuh"
 
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <limits>
 #include <mutex>
@@ -48,7 +50,10 @@ constexpr int kPrepThreads = 1024;
 
 // Byte offsets of the regions inside the scratch array (each 256-byte aligned).
 constexpr size_t Align(size_t b) { return (b + 255) / 256 * 256; }
-constexpr size_t kOffSliceOff = 0;
+// The control block and the slice offsets are neighbours: one copy brings both to the host.
+constexpr size_t kControlBytes = 256;
+constexpr size_t kOffControl = 0;
+constexpr size_t kOffSliceOff = kOffControl + kControlBytes;
 constexpr size_t kOffRowLen = kOffSliceOff + Align(sizeof(int32_t) * (kNoallocMaxSlices + 1));
 constexpr size_t kOffCol = kOffRowLen + Align(sizeof(int32_t) * kNoallocMaxRows);
 constexpr size_t kOffVal = kOffCol + Align(sizeof(int32_t) * kNoallocMaxPositions);
@@ -63,8 +68,7 @@ constexpr size_t kOffP0 = kOffZ + kVec;
 constexpr size_t kOffP1 = kOffP0 + kVec;
 constexpr size_t kOffQ = kOffP1 + kVec;
 constexpr size_t kOffPartials = kOffQ + kVec;
-constexpr size_t kOffControl = kOffPartials + Align(sizeof(double) * 2 * 64 * kNoallocMaxGrid);
-constexpr size_t kScratchBytes = kOffControl + 256;
+constexpr size_t kScratchBytes = kOffPartials + Align(sizeof(double) * 2 * 64 * kNoallocMaxGrid);
 
 // Control block: [0] barrier counter, [1] PCG error flag, [2] set-up error, [3] SELL slots
 // used, [4] inverse diagonal usable; doubles from byte 64: PCG info (status, iterations,
@@ -78,7 +82,14 @@ struct Control {
   int32_t pad[11];
   double info[3];
 };
-static_assert(sizeof(Control) <= 256, "control block");
+static_assert(sizeof(Control) <= kControlBytes, "control block");
+// What the host reads after the set-up kernel.
+struct SetUp {
+  Control control;
+  unsigned char pad[kControlBytes - sizeof(Control)];
+  int32_t slice_off[kNoallocMaxSlices + 1];
+};
+static_assert(offsetof(SetUp, slice_off) == kOffSliceOff - kOffControl, "set-up block");
 
 // The only memory this entry point touches besides the caller's buffers.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -234,19 +245,15 @@ Status NoallocPcg(int32_t n, const int32_t *ro, const int32_t *col, const double
   PrepareKernel<<<1, kPrepThreads, 0, stream>>>(n, ro, col, val, diag, rhs, scratch);
   if (cudaGetLastError() != cudaSuccess)
     return Status::kInternalError;
-  Control control{};
-  if (cudaMemcpyAsync(&control, scratch + kOffControl, sizeof(Control), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess)
-    return Status::kInternalError;
-  if (control.setup_error != kSetupOk)
-    return Status::kInvalidArgument;
   const int n_pad = (n + 31) / 32 * 32;
-  int32_t slice_off[kNoallocMaxSlices + 1]; // the launch sizes its shared memory by these
-  if (cudaMemcpyAsync(slice_off, scratch + kOffSliceOff, sizeof(int32_t) * (n_pad / 32 + 1),
+  SetUp set_up{};
+  if (cudaMemcpyAsync(&set_up, scratch + kOffControl, offsetof(SetUp, slice_off) + sizeof(int32_t) * (n_pad / 32 + 1),
                       cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
       cudaStreamSynchronize(stream) != cudaSuccess)
     return Status::kInternalError;
+  Control &control = set_up.control;
+  if (control.setup_error != kSetupOk)
+    return Status::kInvalidArgument;
   PcgArgs a{};
   a.n = n;
   a.n_pad = n_pad;
@@ -254,7 +261,7 @@ Status NoallocPcg(int32_t n, const int32_t *ro, const int32_t *col, const double
   a.kp = 1;
   a.items = 1;
   a.slice_off = reinterpret_cast<const int32_t *>(scratch + kOffSliceOff);
-  a.host_slice_off = slice_off;
+  a.host_slice_off = set_up.slice_off; // the launch sizes its shared memory by these
   a.row_len = reinterpret_cast<const int32_t *>(scratch + kOffRowLen);
   a.sell_col = reinterpret_cast<const int32_t *>(scratch + kOffCol);
   a.values = reinterpret_cast<const double *>(scratch + kOffVal);

@@ -101,3 +101,9 @@ new, pinned, waits = counted(call)
 @pytest.mark.parametrize("m", [20, 64])
 def test_the_noalloc_solve_uses_no_heap(gpu, counter, m):
     counter(NOALLOC.format(m=m) + "assert new == 0 and pinned == 0, (new, pinned)")
+
+
+@pytest.mark.parametrize("m", [20, 64])
+def test_the_noalloc_solve_waits_three_times(gpu, counter, m):
+    """For the set-up's verdict, for the solve's and for the copy of x."""
+    counter(NOALLOC.format(m=m) + "assert waits == 3, waits")
