@@ -305,18 +305,14 @@ bool PcgWindow(const PcgArgs &args)
 {
   ResidentShape shape;
   const int max_grid = PcgMaxGrid(args.kp);
-  const bool fits = max_grid > 0 && ChooseWindow(args, RowGroups(args, max_grid), &shape) > 0;
-  cudaGetLastError(); // a size beyond the shared-memory limit is not an error here
-  return fits;
+  return max_grid > 0 && ChooseWindow(args, RowGroups(args, max_grid), &shape) > 0;
 }
 
 bool PcgResident(const PcgArgs &args)
 {
   ResidentShape shape;
   const int max_grid = PcgMaxGrid(args.kp);
-  const bool fits = max_grid > 0 && ChooseResident(args, RowGroups(args, max_grid), &shape);
-  cudaGetLastError(); // a size beyond the shared-memory limit is not an error here
-  return fits;
+  return max_grid > 0 && ChooseResident(args, RowGroups(args, max_grid), &shape);
 }
 
 cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t stream)
@@ -362,7 +358,6 @@ cudaError_t LaunchPcg(PcgArgs args, int *grid_out, int *block_out, cudaStream_t 
       *block_out = kPcgThreads;
     return e;
   }
-  cudaGetLastError(); // a size beyond the shared-memory limit is not an error here
   // Wide CTAs (FP64 Jacobi): the same row groups two to a CTA of 1024 threads, one CTA per
   // SM -- the same rows, order and partial sums, so the same bits.
   const bool want_wide = args.block_request == 0 ? WideBlocksEnabled() : args.block_request == 1;
