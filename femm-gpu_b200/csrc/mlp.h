@@ -37,6 +37,7 @@ private:
     float *w1, *b1, *w2, *b2, *w3, *b3;
   };
   Views Split(float *q) const;
+  float *Loss() const { return g_.get() + ParameterCount(); }
   Status EnsureBatch(int batch);
   Status Forward(int batch, const float *x, float *y, cudaStream_t st, const float *target = nullptr);
   Status Backward(int batch, const float *x, cudaStream_t st);
@@ -44,9 +45,8 @@ private:
   int I_ = 0, H_ = 0, O_ = 0;
   int batch_cap_ = 0, loss_partials_ = 0;
   int64_t steps_ = 0, launches_ = 0;
-  DeviceArray<float> p_, g_, m_, v_;
-  DeviceArray<float> x_, t_, h1_, a1_, h2_, a2_, y_, dy_, d2_, d1_, row_loss_ /* tile by tile */, loss_;
-  PinnedArray<float> host_loss_;
+  DeviceArray<float> p_, g_ /* and the loss */, m_, v_;
+  DeviceArray<float> x_, t_, h1_, a1_, h2_, a2_, y_, dy_, d2_, d1_, row_loss_ /* tile by tile */;
 };
 
 } // namespace fg

@@ -80,13 +80,13 @@ class Mlp:
     def loss_gradient(self, x, t):
         x = np.ascontiguousarray(np.atleast_2d(x), np.float32)
         t = np.ascontiguousarray(np.atleast_2d(t), np.float32)
-        g = np.zeros(self.parameter_count, np.float32)
-        loss = C.c_float(0.0)
+        n = self.parameter_count
+        g = np.empty(n + 1, np.float32)  # the loss behind the gradient: one copy brings both
         st = lib().fg_mlp_loss_gradient(self._h, C.c_int32(x.shape[0]), _p(x), _p(t),
-                                        C.byref(loss), _p(g))
+                                        C.c_void_p(g.ctypes.data + n * g.itemsize), _p(g))
         if st:
             raise FgError(st, "fg_mlp_loss_gradient")
-        return loss.value, g
+        return float(g[n]), g[:n]
 
     def train(self, x, t, epochs, batch=256, lr=1e-3, seed=0):
         x = np.ascontiguousarray(np.atleast_2d(x), np.float32)

@@ -1,13 +1,17 @@
 """The host side of short calls: what a call may not ask of the allocator, and how often it
 waits.  A preloaded library counts, for the calling thread, operator new and the runtime
 calls of interest, and passes them on."""
+import ctypes
 import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
+import femm_gpu_b200 as fg
 from conftest import ROOT
+from femm_gpu_b200 import learned
 
 pytestmark = pytest.mark.gpu
 
@@ -107,3 +111,28 @@ def test_the_noalloc_solve_uses_no_heap(gpu, counter, m):
 def test_the_noalloc_solve_waits_three_times(gpu, counter, m):
     """For the set-up's verdict, for the solve's and for the copy of x."""
     counter(NOALLOC.format(m=m) + "assert waits == 3, waits")
+
+
+def test_the_first_gradient_of_a_network_pins_no_memory(gpu, counter):
+    counter("""
+net = learned.Mlp(4, 64, 8, seed=1)
+x, t = np.ones((16, 4), np.float32), np.ones((16, 8), np.float32)
+new, pinned, waits = counted(lambda: net.loss_gradient(x, t))
+assert pinned == 0, pinned
+""")
+
+
+def test_loss_and_gradient_are_the_same_wherever_the_loss_goes(gpu):
+    """Behind the gradient (one copy), elsewhere, or only one of the two asked for."""
+    net = learned.Mlp(4, 40, 5, seed=1)
+    rng = np.random.default_rng(0)
+    x, t = rng.normal(size=(24, 4)).astype(np.float32), rng.normal(size=(24, 5)).astype(np.float32)
+    loss, g = net.loss_gradient(x, t)
+    assert g.shape == (net.parameter_count,) and np.isfinite(loss) and loss > 0.0
+    apart, alone = ctypes.c_float(0.0), ctypes.c_float(0.0)
+    g2, g3 = np.zeros_like(g), np.zeros_like(g)
+    ptr = lambda a: ctypes.c_void_p(a.ctypes.data)  # noqa: E731
+    call = lambda loss, g: fg.lib().fg_mlp_loss_gradient(net._h, ctypes.c_int32(24), ptr(x), ptr(t), loss, g)  # noqa: E731
+    assert call(ctypes.byref(apart), ptr(g2)) == call(ctypes.byref(alone), None) == call(None, ptr(g3)) == 0
+    assert apart.value == alone.value == loss
+    assert np.array_equal(g, g2) and np.array_equal(g, g3)
