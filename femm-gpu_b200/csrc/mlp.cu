@@ -293,11 +293,6 @@ Status Mlp::Create(int inputs, int hidden, int outputs, uint64_t seed)
 {
   if (inputs < 1 || hidden < 1 || outputs < 1 || inputs > 4096 || hidden > 4096 || outputs > 4096)
     return Status::kInvalidArgument;
-  if (cudaFuncSetAttribute(GemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return Status::kGpuUnavailable;
-  }
   I_ = inputs;
   H_ = hidden;
   O_ = outputs;
@@ -306,6 +301,11 @@ Status Mlp::Create(int inputs, int hidden, int outputs, uint64_t seed)
   if ((s = p_.ensure(n)) != Status::kOk || (s = g_.ensure(n + 1)) != Status::kOk ||
       (s = m_.ensure(n)) != Status::kOk || (s = v_.ensure(n)) != Status::kOk)
     return s;
+  if (cudaFuncSetAttribute(GemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return Status::kInternalError;
+  }
   // Uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights and biases from a seeded generator.
   std::mt19937_64 rng(seed);
   std::vector<float> host(n);
