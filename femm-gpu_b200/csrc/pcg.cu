@@ -218,6 +218,11 @@ bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
   const long long ws = args.n_pad / s;
   const bool shared = args.value_item == 0;
   const int per_cta = groups <= sms ? 1 : 2, ctas = (groups + per_cta - 1) / per_cta;
+  // Where a few CTAs own many items' sums, each sums its own one after the other.  32 items on 3
+  // CTAs (81 rows), 11 each: 3.37 ms a solve, streamed 2.75.  On 4 CTAs (121 rows), 8 each: 3.30,
+  // streamed 3.45.  (One or two CTAs add up all items' sums themselves: 0.93, streamed 2.26.)
+  if (ctas > 2 && args.kp > 8 * ctas)
+    return false;
   // The least a CTA can need with the state in shared memory, before looking at the rows.
   int step = 0, entry = 0;
   if (!PcgKernelF64ResidentSteps(args.kp, shared, true, per_cta, &step, &entry) ||
