@@ -26,11 +26,18 @@ namespace fg
 namespace
 {
 
-constexpr int kTileM = 16, kTileN = 32;  // output tile of a CTA
+constexpr int kTileM = 16, kTileN = 32;  // output tile
 constexpr int kGemmThreads = 512, kGemmWarps = kGemmThreads / 32;
-constexpr int kWarpK = 16, kSlab = kGemmWarps * kWarpK; // inner dimension per warp and staged at a time
-constexpr int kPitchA = kTileM + 4, kPitchB = kTileN + 4; // floats of a staged k (16-byte rows)
-constexpr size_t kGemmSmem = sizeof(float) * kSlab * (kPitchA + kPitchB);
+constexpr int kWarpK = 16; // inner dimension per warp
+// A CTA of R row tiles: its warps split into R groups, the inner dimension over the warps of a
+// group.  Floats of a staged k (16-byte rows), inner dimension staged at a time, bytes.
+template <int R> struct GemmShape {
+  static constexpr int kRows = R * kTileM, kSplit = kGemmWarps / R, kSlab = kSplit * kWarpK;
+  static constexpr int kPitchA = kRows + 4, kPitchB = kTileN + 4;
+  static constexpr int kParts = kGemmWarps * (kTileM * kTileN + kTileM); // the warps' tiles and row sums
+  static constexpr int kStaged = kSlab * (kPitchA + kPitchB);
+  static constexpr size_t kSmem = sizeof(float) * (kStaged > kParts ? kStaged : kParts);
+};
 constexpr int kThreads = 256;
 
 enum Epilogue : int { kStore = 0, kBiasGelu = 1, kBias = 2, kGeluGrad = 3, kBiasDelta = 4 };
@@ -69,10 +76,10 @@ struct GemmArgs {
 
 // Stages X(r, k) = X[r * rs + k * ks], r0 <= r < r0 + ROWS, a slab from k0 on, as
 // smem[k][r], zero outside; 16-byte loads along the contiguous direction where aligned.
-template <int ROWS, int PITCH>
+template <int ROWS, int PITCH, int SLAB>
 __device__ __forceinline__ void Stage(float *smem, const float *X, int rs, int ks, int r0, int rows, int k0, int K)
 {
-  const int slab = min(kSlab, (K - k0 + kWarpK - 1) / kWarpK * kWarpK);
+  const int slab = min(SLAB, (K - k0 + kWarpK - 1) / kWarpK * kWarpK);
   const bool aligned = (reinterpret_cast<size_t>(X) & 15) == 0;
   if (rs == 1 && ks % 4 == 0 && aligned) {
     for (int t = threadIdx.x; t < slab * (ROWS / 4); t += kGemmThreads) {
@@ -128,10 +135,16 @@ __device__ __forceinline__ void Stage(float *smem, const float *X, int rs, int k
 // warps multiplies its own 16th of it with 4 x 4 outputs per lane (16 FMAs from two 16-byte
 // shared-memory reads), and the 16 partial tiles are added in warp order.  Measured (B200):
 // loss and gradient of a 4-256-256-64 network at batch 256 through host buffers 318 -> 155 us (two thirds of the rest are copies and the fresh host array).
+//
+// A short inner dimension (the first layer, narrow networks) has no work for 16 warps: with R > 1
+// they take R row tiles instead (RowTiles).  Where R is used, sums and their order are those of
+// R = 1.
+template <int R>
 __global__ void __launch_bounds__(kGemmThreads)
     GemmKernel(GemmArgs g, GemmArgs h, const float *__restrict__ partials, int count, float scale,
                float *__restrict__ loss)
 {
+  using G = GemmShape<R>;
   extern __shared__ __align__(16) float gemm_smem[];
   __shared__ float red[kGemmWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -162,24 +175,26 @@ __global__ void __launch_bounds__(kGemmThreads)
   if (second)
     tile -= g.tiles;
   const GemmArgs &p = second ? h : g;
-  const int m0 = tile / p.tiles_n * kTileM, n0 = tile % p.tiles_n * kTileN;
-  float *const As = gemm_smem, *const Bs = gemm_smem + kSlab * kPitchA;
+  const int m0 = tile / p.tiles_n * G::kRows, n0 = tile % p.tiles_n * kTileN;
+  const int part = warp % G::kSplit; // of the inner dimension; the warp's row tile: warp / kSplit
+  float *const As = gemm_smem, *const Bs = gemm_smem + G::kSlab * G::kPitchA;
   const int mm = (lane >> 3) * 4, nn = (lane & 7) * 4;
   const bool sums = p.row_sum && n0 == 0;
   float acc[4][4] = {}, sum[4] = {};
-  for (int k0 = 0; k0 < p.K; k0 += kSlab) {
+  for (int k0 = 0; k0 < p.K; k0 += G::kSlab) {
     if (k0 > 0)
       __syncthreads();
-    Stage<kTileM, kPitchA>(As, p.A, p.am, p.ak, m0, p.M, k0, p.K);
-    Stage<kTileN, kPitchB>(Bs, p.B, p.bn, p.bk, n0, p.N, k0, p.K);
+    Stage<G::kRows, G::kPitchA, G::kSlab>(As, p.A, p.am, p.ak, m0, p.M, k0, p.K);
+    Stage<kTileN, G::kPitchB, G::kSlab>(Bs, p.B, p.bn, p.bk, n0, p.N, k0, p.K);
     __syncthreads();
-    if (k0 + warp * kWarpK >= p.K)
+    if (k0 + part * kWarpK >= p.K)
       continue;
-    const float *a = As + warp * kWarpK * kPitchA + mm, *b = Bs + warp * kWarpK * kPitchB + nn;
+    const float *a = As + part * kWarpK * G::kPitchA + warp / G::kSplit * kTileM + mm;
+    const float *b = Bs + part * kWarpK * G::kPitchB + nn;
 #pragma unroll
     for (int k = 0; k < kWarpK; ++k) {
-      const float4 av = *reinterpret_cast<const float4 *>(a + k * kPitchA);
-      const float4 bv = *reinterpret_cast<const float4 *>(b + k * kPitchB);
+      const float4 av = *reinterpret_cast<const float4 *>(a + k * G::kPitchA);
+      const float4 bv = *reinterpret_cast<const float4 *>(b + k * G::kPitchB);
       const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -203,35 +218,40 @@ __global__ void __launch_bounds__(kGemmThreads)
     for (int i = 0; i < 4; ++i)
       row[warp * kTileM + mm + i] = sum[i];
   __syncthreads();
-  float v = 0.f;
-#pragma unroll
-  for (int w = 0; w < kGemmWarps; ++w)
-    v += gemm_smem[w * kPart + threadIdx.x];
-  if (sums && threadIdx.x < kTileM && m0 + threadIdx.x < p.M) {
+  if (sums && threadIdx.x < G::kRows && m0 + threadIdx.x < p.M) {
+    const float *w0 = row + threadIdx.x / kTileM * G::kSplit * kTileM + threadIdx.x % kTileM;
     float s = 0.f;
-    for (int w = 0; w < kGemmWarps; ++w)
-      s += row[w * kTileM + threadIdx.x];
+    for (int w = 0; w < G::kSplit; ++w)
+      s += w0[w * kTileM];
     p.row_sum[m0 + threadIdx.x] = s;
   }
-  const int m = m0 + static_cast<int>(threadIdx.x) / kTileN, n = n0 + static_cast<int>(threadIdx.x) % kTileN;
   float l = 0.f;
-  if (m < p.M && n < p.N) {
-    const size_t o = static_cast<size_t>(m) * p.ldc + n;
-    if (p.epilogue == kBiasGelu) {
-      v += p.bias[n];
-      p.aux[o] = v;
-      v = Gelu(v);
-    } else if (p.epilogue == kBias) {
-      v += p.bias[n];
-    } else if (p.epilogue == kGeluGrad) {
-      v *= GeluGrad(p.aux[o]);
-    } else if (p.epilogue == kBiasDelta) {
-      v += p.bias[n];
-      const float e = v - p.target[o];
-      p.delta[o] = e / static_cast<float>(p.M);
-      l = 0.5f * e * e;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < G::kSplit; ++w)
+      v += gemm_smem[(r * G::kSplit + w) * kPart + threadIdx.x];
+    const int m = m0 + r * kTileM + static_cast<int>(threadIdx.x) / kTileN;
+    const int n = n0 + static_cast<int>(threadIdx.x) % kTileN;
+    if (m < p.M && n < p.N) {
+      const size_t o = static_cast<size_t>(m) * p.ldc + n;
+      if (p.epilogue == kBiasGelu) {
+        v += p.bias[n];
+        p.aux[o] = v;
+        v = Gelu(v);
+      } else if (p.epilogue == kBias) {
+        v += p.bias[n];
+      } else if (p.epilogue == kGeluGrad) {
+        v *= GeluGrad(p.aux[o]);
+      } else if (p.epilogue == kBiasDelta) {
+        v += p.bias[n];
+        const float e = v - p.target[o];
+        p.delta[o] = e / static_cast<float>(p.M);
+        l += 0.5f * e * e;
+      }
+      p.C[o] = v;
     }
-    p.C[o] = v;
   }
   if (p.epilogue == kBiasDelta) {
     l = block_sum(l);
@@ -240,7 +260,6 @@ __global__ void __launch_bounds__(kGemmThreads)
   }
 }
 static_assert(kTileM * kTileN == kGemmThreads, "one output per thread in the epilogue");
-static_assert(kGemmSmem >= sizeof(float) * kGemmWarps * (kTileM * kTileN + kTileM), "partial tiles fit the staging");
 
 __global__ void GatherRowsKernel(int rows, int width, const int32_t *__restrict__ index,
                                  const float *__restrict__ src, float *__restrict__ dst)
@@ -279,12 +298,45 @@ GemmArgs Product(int M, int N, int K, const float *A, int am, int ak, const floa
   return g;
 }
 
+template <int R>
+cudaError_t LaunchGemm(GemmArgs g, const GemmArgs &h, cudaStream_t st, const float *partials = nullptr, int count = 0,
+                       float scale = 0.f, float *loss = nullptr)
+{
+  g.tiles = g.tiles_n * ((g.M + GemmShape<R>::kRows - 1) / GemmShape<R>::kRows);
+  GemmKernel<R><<<g.tiles + h.tiles + (loss ? 1 : 0), kGemmThreads, GemmShape<R>::kSmem, st>>>(g, h, partials, count,
+                                                                                              scale, loss);
+  return cudaGetLastError();
+}
+
+// Row tiles per CTA of a single product whose epilogue writes no sums: the fewest that leave one
+// wave (two CTAs per SM, by registers) and a part of the inner dimension to every warp.  A CTA per
+// tile and two to seven waves of them were slower than 32 x 32 tiles of 256 threads at narrow
+// widths.  Forward pass through host buffers, us: 32 x 32 tiles, a CTA per tile, by this rule:
+//   4-32-32-4:     8,192 rows  57  68  59,   32,768 rows 132 172 132
+//   4-48-48-8:     4,096 rows  52  63  53,   32,768 rows 189 250 182
+//   4-128-128-16:  4,096 rows  96  88  75,   32,768 rows 455 447 320
+int RowTiles(const GemmArgs &g)
+{
+  constexpr int kWave = 2 * 148;
+  int tiles = 1;
+  if (g.epilogue == kBiasGelu || g.epilogue == kBias)
+    for (const int r : {2, 4, 16})
+      if (g.K <= kGemmWarps / r * kWarpK && g.tiles > kWave * tiles)
+        tiles = r;
+  return tiles;
+}
+
 // g and optionally h (h.tiles = 0: none); with loss, also the sum of `count` partials.
 cudaError_t Gemm(const GemmArgs &g, const GemmArgs &h, cudaStream_t st, const float *partials = nullptr,
                  int count = 0, float scale = 0.f, float *loss = nullptr)
 {
-  GemmKernel<<<g.tiles + h.tiles + (loss ? 1 : 0), kGemmThreads, kGemmSmem, st>>>(g, h, partials, count, scale, loss);
-  return cudaGetLastError();
+  if (h.tiles == 0 && !loss)
+    switch (RowTiles(g)) {
+    case 16: return LaunchGemm<16>(g, h, st);
+    case 4: return LaunchGemm<4>(g, h, st);
+    case 2: return LaunchGemm<2>(g, h, st);
+    }
+  return LaunchGemm<1>(g, h, st, partials, count, scale, loss);
 }
 
 } // namespace
@@ -301,8 +353,8 @@ Status Mlp::Create(int inputs, int hidden, int outputs, uint64_t seed)
   if ((s = p_.ensure(n)) != Status::kOk || (s = g_.ensure(n + 1)) != Status::kOk ||
       (s = m_.ensure(n)) != Status::kOk || (s = v_.ensure(n)) != Status::kOk)
     return s;
-  if (cudaFuncSetAttribute(GemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)) !=
-      cudaSuccess) {
+  if (cudaFuncSetAttribute(GemmKernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(GemmShape<1>::kSmem)) != cudaSuccess) {
     cudaGetLastError();
     return Status::kInternalError;
   }
