@@ -32,3 +32,18 @@ def test_large_batches_give_the_bits_of_small_ones(gpu, I, H, O, B):
     assert np.array_equal(y, parts)
     y64, _ = M.forward(net.get_parameters(), x, I, H, O)
     assert rel(y, y64) <= 1e-5
+
+
+@pytest.mark.parametrize("I, H, O, B", [(4, 300, 50, 64), (5, 30, 7, 33), (3, 257, 1, 17), (4, 48, 8, 1), (1, 1, 1, 600),
+                                        (4, 520, 96, 40), (4, 64, 8, 5000)])
+def test_gradients_match_the_oracle(gpu, I, H, O, B):
+    net = learned.Mlp(I, H, O, seed=5)
+    p = net.get_parameters()
+    x, t = data(B, I, O, seed=B)
+    loss, g = net.loss_gradient(x, t)
+    loss64, g64 = M.loss_gradient(p, x, t, I, H, O)
+    assert abs(loss - loss64) <= 1e-5 * loss64
+    o = 0
+    for n in (H * I, H, H * H, H, O * H, O):
+        assert rel(g[o:o + n], g64[o:o + n]) <= 1e-4, (o, n)
+        o += n
