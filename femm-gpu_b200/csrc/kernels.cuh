@@ -101,8 +101,8 @@ struct PcgArgs {
   // number of row groups), 2 CTAs of 512.  Both shapes give the same bits.
   int32_t block_request;
   // Resident form (FP64 Jacobi; pcg_resident.cuh): 0 wherever each CTA's share fits in
-  // shared memory (needs host_slice_off), 2 off.  The same bits either way.  row_groups and
-  // resident_offset are set by LaunchPcg.
+  // shared memory (needs host_slice_off), 1 off, 2 off and the window form too.  The same bits
+  // either way.  row_groups and resident_offset are set by LaunchPcg.
   int32_t resident_request, row_groups, resident_offset;
   // Window form (FP64 Jacobi; pcg_window.cuh): window_request 1 asks for it where the resident
   // form does not fit and this one does (the same bits again); bandwidth: the operator's

@@ -207,7 +207,7 @@ struct ResidentShape {
 // memory, the operator's values beside it or, where they do not fit, in L2.
 bool ChooseResident(const PcgArgs &args, int groups, ResidentShape *out)
 {
-  if (args.resident_request == 2 || args.precision != 0 || args.blocks || args.one_reduction ||
+  if (args.resident_request != 0 || args.precision != 0 || args.blocks || args.one_reduction ||
       !args.host_slice_off)
     return false;
   int device = 0, sms = 0;

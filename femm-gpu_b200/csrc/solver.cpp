@@ -125,6 +125,7 @@ Status Plan::Create(HostModel model, const fg_plan_options &options)
   from_iterate_ = (options_.flags & FG_PLAN_PCG_FROM_ITERATE) != 0;
   one_reduction_ = (options_.flags & FG_PLAN_PCG_ONE_REDUCTION) != 0;
   streamed_ = (options_.flags & FG_PLAN_PCG_STREAMED) != 0;
+  windowed_ = (options_.flags & FG_PLAN_PCG_WINDOW) != 0;
   if (one_reduction_ && (options_.precision != FG_PRECISION_FP64 || block_size() != 0))
     return Status::kUnsupportedFeature;
   if (host_only_)
@@ -413,7 +414,8 @@ bool TuningEnabled()
 cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t stream)
 {
   const int key = a.kp * 1000 + a.precision * 100 + (a.blocks ? a.block_size : 0) + (a.value_item ? 0 : 100000);
-  a.resident_request = streamed_ ? 2 : 0;
+  a.resident_request = streamed_ ? 2 : (windowed_ ? 1 : 0);
+  a.window_request = windowed_ ? 1 : 0;
   auto it = shapes_.find(key);
   if (it == shapes_.end() && TuningEnabled()) {
     fg_pcg_shape sh{};
@@ -457,7 +459,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         const int ring = c % 2 == 0 ? 1 : 2, cache = c == 2 || c == 3 ? 1 : 2;
         if (c < 5 ? ring == 1 && !ring_possible : !window)
           continue;
-        t.resident_request = c < 5 ? 2 : 0;
+        t.resident_request = c < 5 ? 2 : 1;
         t.window_request = c < 5 ? 0 : 1;
         t.ring_request = ring;
         t.col_cache_request = cache;
@@ -491,7 +493,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         sh.column_cache = c == 2 || c == 3 ? 1 : 0;
         sh.threads_per_block = c == 4 ? 1024 : 512;
       }
-    sh.resident = resident ? 1 : (window_us > 0.0 && window_us < best ? 2 : 0);
+    sh.resident = resident ? 1 : (window_us > 0.0 && (windowed_ || window_us < best) ? 2 : 0);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (sh.candidates > 0)
@@ -816,6 +818,7 @@ Status Plan::EnsureLanes(int lanes)
     lane->chunk_cap_ = chunk_cap_;
     lane->from_iterate_ = from_iterate_;
     lane->streamed_ = streamed_;
+    lane->windowed_ = windowed_;
     lane->host_only_ = true;
     Status s = lane->AttachDevice();
     if (s != Status::kOk)

@@ -150,6 +150,7 @@ private:
   bool from_iterate_ = false; // FG_PLAN_PCG_FROM_ITERATE
   bool one_reduction_ = false; // FG_PLAN_PCG_ONE_REDUCTION
   bool streamed_ = false; // FG_PLAN_PCG_STREAMED
+  bool windowed_ = false; // FG_PLAN_PCG_WINDOW
   int32_t bandwidth_ = 0; // largest |row - column| of the pattern
   int pcg_grid_cap_ = 0;
   int chunk_cap_ = kMaxItems; // items per batched launch

@@ -34,6 +34,7 @@ PLAN_HOST_ONLY = 1
 PLAN_PCG_FROM_ITERATE = 2
 PLAN_PCG_ONE_REDUCTION = 4
 PLAN_PCG_STREAMED = 8
+PLAN_PCG_WINDOW = 16
 
 EXPORTED = [
     "fg_production_options", "fg_status_name", "fg_abi_version", "fg_plan_create",
@@ -218,7 +219,7 @@ class Plan:
 
     def __init__(self, model: Model, preconditioner: int = 0, block_size: int = 8,
                  precision: int = 0, host_only: bool = False, from_iterate: bool = False,
-                 one_reduction: bool = False, streamed: bool = False):
+                 one_reduction: bool = False, streamed: bool = False, window: bool = False):
         self.model = model
         L = lib()
         self._keep = []
@@ -248,7 +249,8 @@ class Plan:
             self._keep.append(ages)
             fm.air_gap_count, fm.air_gap_elements = len(model.ages), C.cast(ages, C.c_void_p)
         flags = ((PLAN_HOST_ONLY if host_only else 0) | (PLAN_PCG_FROM_ITERATE if from_iterate else 0) |
-                 (PLAN_PCG_ONE_REDUCTION if one_reduction else 0) | (PLAN_PCG_STREAMED if streamed else 0))
+                 (PLAN_PCG_ONE_REDUCTION if one_reduction else 0) | (PLAN_PCG_STREAMED if streamed else 0) |
+                 (PLAN_PCG_WINDOW if window else 0))
         opts = FgPlanOptions(preconditioner, block_size, precision, flags)
         self._h = C.c_void_p()
         status = L.fg_plan_create(C.byref(fm), C.byref(opts), C.byref(self._h))

@@ -138,13 +138,18 @@ typedef struct fg_plan_options {
  * (the true-residual check); results agree with the default form within the solve's
  * tolerance, not bit for bit.  With block-Jacobi or mixed precision fg_plan_create
  * returns FG_UNSUPPORTED_FEATURE. */
-/* FG_PLAN_PCG_STREAMED: the plan's PCG launches never keep their share of the system in
- * shared memory (the resident form, chosen where it fits); same results bit for bit. */
+/* FG_PLAN_PCG_STREAMED: the plan's PCG launches take neither the resident form (each CTA's
+ * share of the system in shared memory, chosen where it fits) nor the window form (the SpMV's
+ * operand in a sliding window in shared memory, chosen where it fits and is timed faster).
+ * FG_PLAN_PCG_WINDOW: FP64 Jacobi launches with an operator per item take the window form
+ * wherever it fits, also in place of the resident form and whatever the times.  The results
+ * are the same bits in every form; the flags are for tests and comparison. */
 enum {
   FG_PLAN_HOST_ONLY = 1,
   FG_PLAN_PCG_FROM_ITERATE = 2,
   FG_PLAN_PCG_ONE_REDUCTION = 4,
-  FG_PLAN_PCG_STREAMED = 8
+  FG_PLAN_PCG_STREAMED = 8,
+  FG_PLAN_PCG_WINDOW = 16
 };
 
 /* NonlinearOptions (gpu_solver/src/physics/nonlinear_model.h:102-109). */

@@ -26,3 +26,92 @@ def test_few_ctas_with_many_items_are_left_to_the_streamed_form(gpu, m, items, r
     plans = [fg.Plan(model, streamed=s) for s in (False, True)]
     same(*[p.solve(currents) for p in plans])
     assert plans[0].pcg_shapes()[0]["resident"] == resident
+
+
+def window_rows(plan, items):
+    """Shared-memory bytes of the window form's ring and of q beside it, as the launch sizes them."""
+    ro, col = plan.symbolic()[:2]
+    bandwidth = int(np.abs(np.repeat(np.arange(plan.rows), np.diff(ro)) - col).max())
+    kp = 1 << (items - 1).bit_length()
+    step = 32 * min(kp, 2) // kp  # rows of a warp-step
+    steps = -(-plan.rows // 32) * 32 // step
+    groups = min(-(-steps // 16), 296)
+    most = max(steps * min(groups, 2 * c + 2) // groups - steps * 2 * c // groups for c in range((groups + 1) // 2))
+    return (2 * bandwidth + 4 * 16 * step) * kp * 8, most * step * kp * 8
+
+
+MODELS = {"square30": lambda: meshes.square_nonlinear(m=30, seed=5), "square12": lambda: meshes.square_nonlinear(m=12, seed=5),
+          "sector2400": lambda: meshes.annular_sector(40, 60), "sector": meshes.annular_sector,
+          "plunger": meshes.axisymmetric_plunger,
+          "wide_rows": lambda: meshes.sliding_band_machine(nr=40, nt=30, rotor_deg=7.3)}
+
+
+@pytest.mark.parametrize("name, items", [
+    ("square12", 1), ("square12", 13),  # one round, one CTA
+    ("square30", 1), ("square30", 2), ("square30", 3), ("square30", 8), ("square30", 16), ("square30", 32),
+    ("sector2400", 1), ("sector2400", 7),  # odd numbers of row groups: 5, 19
+    ("wide_rows", 1), ("wide_rows", 2), ("wide_rows", 3), ("wide_rows", 5), ("wide_rows", 16),  # rows of 20 entries
+    ("sector", 4), ("sector", 16), ("sector", 32), ("plunger", 1), ("plunger", 9), ("plunger", 32)])
+def test_the_window_form_where_it_is_asked_for(gpu, name, items):
+    model = MODELS[name]()
+    plans = [fg.Plan(model, window=True), fg.Plan(model, streamed=True)]
+    currents = meshes.seeded_currents(items, model.circuit_count, 15.0, seed=items)
+    currents[::3] *= 1e-3  # linear items beside saturated ones
+    options = fg.production_options(max_newton_iterations=6, recover_nonconvergence=0)
+    same(*[p.solve(currents, options=options) for p in plans])
+    assert plans[0].pcg_shapes()[0]["window"] and not plans[1].pcg_shapes()[0]["window"]
+    ring, q = window_rows(plans[0], items)
+    in_shared = ring + q <= 220 * 1024
+    assert in_shared == (not (items == 32 and name in ("sector", "plunger")))  # both places are tried
+
+
+@pytest.mark.parametrize("budget", [0, 1, 2, 7, 8])
+def test_window_form_iteration_budgets(gpu, budget):
+    model = MODELS["sector2400"]()
+    plans = [fg.Plan(model, window=True), fg.Plan(model, streamed=True)]
+    currents = meshes.seeded_currents(5, model.circuit_count, 15.0, seed=1)
+    options = fg.production_options(max_newton_iterations=2, max_linear_iterations=budget, recover_nonconvergence=0)
+    same(*[p.solve(currents, options=options) for p in plans])
+    assert plans[0].pcg_shapes()[0]["window"]
+
+
+def linear_systems(plan, items, shared):
+    """Operators and right-hand sides with a zero one, one that is not finite and (an operator per
+    item) an indefinite operator; then subnormal values, whose reciprocals overflow, so that the
+    Jacobi step divides."""
+    vals, _, _ = plan.assemble(np.zeros((1, plan.N)), np.ones((1, 3)), 0)
+    rng = np.random.default_rng(11)
+    rhs = rng.normal(size=(6, plan.rows))
+    rhs[1] = 0.0
+    rhs[2, 100] = np.nan
+    vals = vals * (1.0 + 0.1 * np.arange(6))[:, None]
+    if not shared:
+        vals[3] *= -1.0
+    for scale in (1.0, 1e-309):
+        if items == 1:
+            for i in range(4):
+                yield scale * vals[i] if shared else scale * vals[i:i + 1], rhs[i:i + 1]
+        else:
+            yield scale * vals[0] if shared else scale * vals, rhs
+
+
+# Systems of each form and of its variants: the window form (small, and with several rounds),
+# two row groups per CTA with the values in shared memory and in L2, an odd number of groups, and
+# one operator for all items.
+@pytest.mark.parametrize("form, m, items, shared, grid", [
+    ("window", 30, 6, False, 4), ("window", 30, 1, False, 1), ("window", 250, 6, False, 148),
+    ("resident", 140, 6, False, 76), ("resident", 277, 1, False, 75), ("resident", 140, 6, True, 76),
+    ("resident", 208, 6, True, 148), ("resident", 277, 1, True, 75)])
+@pytest.mark.parametrize("tol, maxit", [(1e-10, 2000), (3e-16, 120), (1e-10, 0), (1e-10, 3)])
+def test_linear_solves_give_the_streamed_bits(gpu, form, m, items, shared, grid, tol, maxit):
+    """Restarts from the true residual (a tolerance at the rounding level), budgets, zero and
+    non-finite right-hand sides, an indefinite operator, and the dividing preconditioner."""
+    model = meshes.square_nonlinear(m=m, seed=5)
+    plans = [fg.Plan(model, window=form == "window"), fg.Plan(model, streamed=True)]
+    for operator, rhs in linear_systems(plans[0], items, shared):
+        res = [p.pcg(operator, rhs, tol=tol, maxit=maxit, shared=shared) for p in plans]
+        assert np.array_equal(res[0][0], res[1][0], equal_nan=True)
+        for x, y in zip(res[0][1], res[1][1]):
+            assert (x.status, x.iterations) == (y.status, y.iterations)
+            assert x.residual_l2 == y.residual_l2 or (np.isnan(x.residual_l2) and np.isnan(y.residual_l2))
+    assert plans[0].pcg_shapes()[0][form] and plans[0].last_timing().pcg_grid == grid
