@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import femm_gpu_b200 as fg
+import oracle as O
 from femm_gpu_b200 import meshes
 
 pytestmark = pytest.mark.gpu
@@ -115,3 +116,47 @@ def test_linear_solves_give_the_streamed_bits(gpu, form, m, items, shared, grid,
             assert (x.status, x.iterations) == (y.status, y.iterations)
             assert x.residual_l2 == y.residual_l2 or (np.isnan(x.residual_l2) and np.isnan(y.residual_l2))
     assert plans[0].pcg_shapes()[0][form] and plans[0].last_timing().pcg_grid == grid
+
+
+@pytest.mark.parametrize("streamed", [False, True])
+def test_small_linear_solves_match_the_oracle(gpu, streamed):
+    """The streamed form at sizes that a plan gives to the resident one, beside it."""
+    model = meshes.square_nonlinear(m=30, seed=5)
+    plan = fg.Plan(model, streamed=streamed)
+    s = O.assemble(model, np.zeros(model.node_count), [3.0, -5.0, 8.0], 0)
+    nan = s.rhs.copy()
+    nan[17] = np.nan
+    for values, rhs, tol, maxit in ((s.val, s.rhs, 1e-10, 2000), (s.val, s.rhs, 1e-10, 3), (s.val, s.rhs, 1e-10, 0),
+                                    (s.val, 0.0 * s.rhs, 1e-10, 2000), (s.val, nan, 1e-10, 2000),
+                                    (-s.val, s.rhs, 1e-10, 2000), (s.val, s.rhs, 1e-14, 2000)):
+        system = O.csr_system(s.off, s.col, values, rhs)
+        status, x, its, res = O.pcg(system, rhs=rhs, tol=tol, maxit=maxit)
+        got, info = plan.pcg(values[None, :], rhs, tol=tol, maxit=maxit)
+        assert info[0].status == status
+        if status == 0:
+            assert abs(info[0].iterations - its) <= 1 + its // 50
+            assert np.linalg.norm(got[0] - x) <= 1e-6 * np.linalg.norm(x)
+        if maxit in (0, 3):
+            assert info[0].iterations == its == maxit
+            assert abs(info[0].residual_l2 - res) <= 1e-9 * res
+    assert plan.pcg_shapes()[0]["resident"] is not streamed
+
+
+def test_streamed_launch_shapes_leave_results_bitwise_unchanged(gpu, monkeypatch):
+    """The shapes that the autotuner chooses from on a plan that runs them: tuned, untuned, and in
+    CTAs of 1024 threads."""
+    model = meshes.square_nonlinear(m=60, seed=3)
+    currents = meshes.seeded_currents(8, 3, 20.0, seed=13)
+    tuned = fg.Plan(model, streamed=True)
+    r = [tuned.solve(currents)]
+    shape = tuned.pcg_shapes()[0]
+    assert not shape["resident"] and not shape["window"] and shape["candidates"] == 5
+    assert tuned.last_timing().pcg_block == shape["threads_per_block"]
+    monkeypatch.setenv("FG_PCG_TUNE", "0")
+    for block in ("512", "1024"):
+        monkeypatch.setenv("FG_PCG_BLOCK", block)
+        plan = fg.Plan(model, streamed=True)
+        r.append(plan.solve(currents))
+        assert plan.pcg_shapes() == [] and plan.last_timing().pcg_block == int(block)
+    same(r[0], r[1])
+    same(r[0], r[2])
