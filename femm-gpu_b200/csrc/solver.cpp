@@ -494,6 +494,10 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         sh.threads_per_block = c == 4 ? 1024 : 512;
       }
     sh.resident = resident ? 1 : (window_us > 0.0 && (windowed_ || window_us < best) ? 2 : 0);
+    if (sh.resident) { // 512 threads, neither ring nor cache
+      sh.value_ring = sh.column_cache = 0;
+      sh.threads_per_block = 512;
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (sh.candidates > 0)

@@ -350,11 +350,13 @@ int fg_plan_attach_device(fg_plan *plan);
 int fg_plan_last_timing(const fg_plan *plan, fg_timing *timing);
 
 /* The plan's PCG launch shapes.  At the first PCG launch of each (items per launch,
- * precision, block size) a plan times its candidate shapes -- the operator-value ring in
- * shared memory on / off, the per-CTA column-index cache off / on -- on the system it is
- * about to solve (a short run of the same kernel), and keeps the fastest for every later
- * launch of that key.  Neither knob changes any arithmetic: results are the same bits
- * whatever the choice.  No counterpart in the reference (its kernel shape is fixed,
+ * precision, block size, one operator or one per item) a plan times its candidate shapes of
+ * the streamed kernel -- the operator-value ring in shared memory on / off, the per-CTA
+ * column-index cache off / on, CTAs of 512 or 1024 threads -- and, where it fits, the window
+ * form, on the system it is about to solve (a short run of the same kernel), and keeps the
+ * fastest for every later launch of that key.  The resident form is taken wherever it fits; the
+ * times are then for information.  None of this changes any arithmetic: results are the same
+ * bits whatever the choice.  No counterpart in the reference (its kernel shape is fixed,
  * gpu_solver/src/solvers/options.cpp:43-53).  FG_PCG_TUNE=0 in the environment keeps the
  * defaults.  Writes at most `capacity` entries; returns the number of tuned keys. */
 typedef struct fg_pcg_shape {
@@ -363,13 +365,13 @@ typedef struct fg_pcg_shape {
   int32_t block_size;   /* 0 Jacobi, 8 or 32 block-Jacobi */
   int32_t value_ring;   /* 1 chosen on, 0 off */
   int32_t column_cache; /* 1 chosen on, 0 off */
-  int32_t candidates;   /* shapes timed (those the kernel shape admits) */
+  int32_t candidates;   /* streamed shapes timed (those the kernel shape admits) */
   /* per candidate: [0..3] 512-thread CTAs, ring on / off x cache off / on; [4] 1024-thread
    * CTAs (two row groups each, FP64 Jacobi with an even number of row groups), ring on,
    * cache off; 0 if not timed */
   double us_per_iteration[5];
-  int32_t threads_per_block; /* the fastest of these: 512 or 1024 (the same bits either way) */
-  int32_t resident;          /* not among these and used instead: 1 the resident form, 2 the window form */
+  int32_t threads_per_block; /* the chosen CTA shape: 512 or 1024 (the same bits either way) */
+  int32_t resident;          /* the form: 0 streamed, 1 resident, 2 window (neither has ring or cache) */
 } fg_pcg_shape;
 int fg_plan_pcg_shapes(const fg_plan *plan, int32_t capacity, fg_pcg_shape *shapes);
 

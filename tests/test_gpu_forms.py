@@ -160,3 +160,12 @@ def test_streamed_launch_shapes_leave_results_bitwise_unchanged(gpu, monkeypatch
         assert plan.pcg_shapes() == [] and plan.last_timing().pcg_block == int(block)
     same(r[0], r[1])
     same(r[0], r[2])
+
+
+@pytest.mark.parametrize("form", ["resident", "window"])
+def test_the_reported_shape_is_the_one_that_runs(gpu, form):
+    plan = fg.Plan(meshes.square_nonlinear(m=60, seed=3), window=form == "window")
+    plan.solve(meshes.seeded_currents(8, 3, 20.0, seed=13))
+    shape = plan.pcg_shapes()[0]
+    assert shape[form] and shape["threads_per_block"] == plan.last_timing().pcg_block == 512
+    assert not shape["value_ring"] and not shape["column_cache"] and shape["candidates"] == 5
