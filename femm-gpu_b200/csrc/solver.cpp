@@ -398,10 +398,13 @@ Status Plan::RunPcg(int kp, int items, uint32_t mask, double tolerance, int max_
 
 namespace
 {
-// CG iterations of each timed candidate launch, and rounds over the candidates.  Where the
-// resident form runs instead of them, one short round reports their times.
+// CG iterations of each timed candidate launch, rounds over the candidates, and how far (times)
+// behind the best so far a candidate is left out of the next round: two launches of one shape
+// differ by 2 % at most.  Where the resident form runs instead of them, one short round without
+// a warm-up reports their times.
 constexpr int kTuneIterations = 64;
 constexpr int kTuneRounds = 2;
+constexpr double kTuneBehind = 1.1;
 constexpr int kTuneIterationsResident = 16;
 
 bool TuningEnabled()
@@ -450,14 +453,19 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
     t.trace = nullptr;
     t.block_request = 2;
     t.resident_request = 2;
-    if (LaunchPcg(t, nullptr, nullptr, stream) != cudaSuccess)
-      cudaGetLastError();
-    else
-      timing_.kernel_launches += 1;
+    if (!resident) {
+      if (LaunchPcg(t, nullptr, nullptr, stream) != cudaSuccess)
+        cudaGetLastError();
+      else
+        timing_.kernel_launches += 1;
+    }
+    double fastest = 0.0; // of all candidates so far
     for (int round = 0; round < rounds; ++round)
       for (int c = 0; c < 6; ++c) {
         const int ring = c % 2 == 0 ? 1 : 2, cache = c == 2 || c == 3 ? 1 : 2;
         if (c < 5 ? ring == 1 && !ring_possible : !window)
+          continue;
+        if (round > 0 && (c < 5 ? sh.us_per_iteration[c] : window_us) > kTuneBehind * fastest)
           continue;
         t.resident_request = c < 5 ? 2 : 1;
         t.window_request = c < 5 ? 0 : 1;
@@ -476,6 +484,7 @@ cudaError_t Plan::LaunchShaped(PcgArgs a, int *grid, int *block, cudaStream_t st
         if (c == 4 && threads != 1024)
           continue; // the launch fell back to 512 threads: not a candidate of its own
         const double us = 1e3 * ms / iterations;
+        fastest = fastest == 0.0 ? us : std::min(fastest, us);
         if (c == 5)
           window_us = window_us == 0.0 ? us : std::min(window_us, us);
         else if (sh.us_per_iteration[c] == 0.0) {

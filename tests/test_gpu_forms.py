@@ -169,3 +169,17 @@ def test_the_reported_shape_is_the_one_that_runs(gpu, form):
     shape = plan.pcg_shapes()[0]
     assert shape[form] and shape["threads_per_block"] == plan.last_timing().pcg_block == 512
     assert not shape["value_ring"] and not shape["column_cache"] and shape["candidates"] == 5
+
+
+@pytest.mark.parametrize("m, form, most", [(60, "resident", 5), (354, "window", 9)])
+def test_trials_of_the_first_solve(gpu, m, form, most):
+    """No warm-up where the times are only reported; no second trial of a candidate that was clearly
+    behind in the first (five streamed shapes against the window form, a fifth faster)."""
+    plan = fg.Plan(meshes.square_nonlinear(m=m, seed=3))
+    currents = meshes.seeded_currents(8, 3, 20.0, seed=13)
+    options = fg.production_options(max_newton_iterations=2, max_linear_iterations=100, recover_nonconvergence=0)
+    launches = []
+    for _ in range(2):
+        plan.solve(currents, options=options)
+        launches.append(plan.last_timing().kernel_launches)
+    assert plan.pcg_shapes()[0][form] and 0 < launches[0] - launches[1] <= most
