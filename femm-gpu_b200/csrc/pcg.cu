@@ -176,11 +176,12 @@ int PcgMaxGrid(int kp)
 
 size_t PcgPartialsDoubles(int kp, int grid)
 {
-  // Double-buffered sums of the barrier-based reductions; the resident form's eight mailbox
-  // buffers of partials (at most 64 x 64 pairs where every CTA gets them) and result lines.
+  // Double-buffered sums of the barrier-based reductions, then eight mailbox buffers of two sums
+  // per item and row group and a line of results per CTA (pcg_resident.cuh); or the streamed
+  // kernels' buffers (at most three sums of 32 items).
   const size_t k = static_cast<size_t>(kp), g = static_cast<size_t>(grid);
-  const size_t partials = std::max<size_t>(2 * k * g, 2 * 64 * 64), line = std::max<size_t>(2 * k, 16);
-  return std::max<size_t>(4 * k * g + 8 * (partials + g * line), 2 * 96 * g);
+  const size_t line = std::max<size_t>(2 * k, 16);
+  return std::max<size_t>(4 * k * g + 8 * (2 * k * g + g * line), 2 * 96 * g);
 }
 
 namespace

@@ -255,8 +255,7 @@ cudaError_t LaunchPostprocess(const PostprocessDevice &p, cudaStream_t stream)
   switch (ItemsTogether(p.items)) {
   case 1: PostprocessKernel<1><<<ctas, kThreads, 0, stream>>>(p); break;
   case 2: PostprocessKernel<2><<<ctas, kThreads, 0, stream>>>(p); break;
-  case 4: PostprocessKernel<4><<<ctas, kThreads, 0, stream>>>(p); break;
-  default: PostprocessKernel<8><<<ctas, kThreads, 0, stream>>>(p); break;
+  default: PostprocessKernel<4><<<ctas, kThreads, 0, stream>>>(p); break;
   }
   return cudaGetLastError();
 }
