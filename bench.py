@@ -119,13 +119,14 @@ def cpu_model():
     return "unknown"
 
 
-def traffic_per_cg_iteration(workload):
-    """DRAM bytes per CG iteration of the PCG kernel from the committed ncu capture of that
-    workload (profiles/traffic.json; the capture's command is in the profile beside it)."""
+def traffic_per_cg_iteration(workload, form):
+    """DRAM bytes per CG iteration of the PCG kernel that runs in this form from the committed
+    ncu capture of that workload (profiles/traffic.json; the capture's command is in the profile
+    beside it)."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
     if not os.path.exists(path):
         return None, None
-    d = json.load(open(path)).get(workload)
+    d = json.load(open(path)).get(workload if form == "streamed" else f"{workload}_{form}")
     return (float(d["dram_bytes_per_cg_iteration"]), d["profile"]) if d else (None, None)
 
 
@@ -332,10 +333,11 @@ def run_ours(args, world, rank, local):
     ms = max_over_ranks(sum(e0.elapsed_time(e1) for e0, e1 in zip(ev0, ev1)), world, dev)
     value = weak_value(world, k, args.steps, ms / 1e3)
 
-    # Roofline of the dominant kernel (the cooperative PCG).
+    # Roofline of the dominant kernel (the cooperative PCG), in the form that ran.
     n, nnz = plan.rows, plan.nnz
-    per_item = 8.0 * nnz + 104.0 * n  # values + vector traffic of one item's iteration
-    shared = 4.0 * nnz + 4.0 * (n + 1)  # column indices + row structure, once per iteration
+    form = pcg_form(plan, k, 0)
+    per_item = pcg_bytes_per_item_iteration(n, nnz, 0, 0, form)
+    shared = pcg_shared_bytes(n, nnz, form)
     alg_bytes = item_its * per_item + pcg_its * shared
     achieved = alg_bytes / (pcg_ms / 1e3) / 1e9 if pcg_ms > 0 else 0.0
     peak, peak_kind = peaks()
@@ -343,7 +345,7 @@ def run_ours(args, world, rank, local):
     # per launch of this run.
     traffic, traffic_src = None, None
     if args.mesh == MESH_M and k == 8:
-        per_it, traffic_src = traffic_per_cg_iteration("square500_items8")
+        per_it, traffic_src = traffic_per_cg_iteration("square500_items8", form)
         if per_it is not None:
             traffic = per_it * pcg_its / max(1, newton)
 
@@ -367,8 +369,8 @@ def run_ours(args, world, rank, local):
         "items_per_step": k, "solver": "fp64 Jacobi PCG (the drop-in form)",
         "e2e": e2e,
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic, "kernel": "PcgKernel",
+        "roofline": {"bound": "latency" if form == "resident" else "hbm", "achieved": achieved, "peak": peak,
+                     "unit": "GB/s", "frac": achieved / peak, "traffic": traffic, "kernel": PCG_KERNELS[form],
                      "traffic_source": (f"ncu capture of this workload, DRAM bytes per CG iteration x "
                                         f"iterations per launch ({traffic_src})") if traffic_src else None,
                      "algorithmic_bytes_per_launch": alg_bytes / max(1, newton),
@@ -785,11 +787,37 @@ def reference_gpu_form(mesh=MESH_M, items=8):
     return out
 
 
-def pcg_bytes_per_item_iteration(n, nnz, precision, block):
-    """Algorithmic bytes of one item's CG iteration (values + the 13 vector passes), FP64
-    or the FP32 inner form; block-Jacobi adds the block inverses' read."""
+PCG_KERNELS = {"streamed": "PcgKernel", "resident": "PcgResidentKernel / PcgResidentStepsKernel",
+               "window": "PcgWindowKernel"}
+
+
+def pcg_form(plan, items, precision):
+    """The form of the plan's PCG launches of that many items (up to 32 per launch), as its tuner
+    reports it: "streamed", "resident" or "window"."""
+    kp = 1 << (min(items, 32) - 1).bit_length()
+    for shape in plan.pcg_shapes():
+        if shape["items"] == kp and shape["precision"] == precision:
+            return "resident" if shape["resident"] else "window" if shape["window"] else "streamed"
+    return "streamed"
+
+
+def pcg_bytes_per_item_iteration(n, nnz, precision, block, form="streamed"):
+    """Algorithmic bytes of one item's CG iteration, FP64 or the FP32 inner form.  Streamed: the
+    values and 13 vector passes; block-Jacobi adds the block inverses' read.  Window (q beside its
+    ring in shared memory): the values and nine passes -- z, p read and p written; r read and
+    written, 1/d read, z written; and, every other iteration, x read and written and two p read.
+    Resident: z, written once; the rest stays on chip."""
     w = 8 if precision == 0 else 4
+    if form == "resident":
+        return w * n
+    if form == "window":
+        return w * nnz + 9 * w * n
     return w * nnz + 13 * w * n + (w * block * n if block else 0)
+
+
+def pcg_shared_bytes(n, nnz, form="streamed"):
+    """Column indices and row structure, once per CG iteration for all items."""
+    return 0.0 if form == "resident" else 4.0 * nnz + 4.0 * (n + 1)
 
 
 def pcg_launch_form(dev, stream, m, k, iterations, launches, one_reduction):
@@ -797,8 +825,8 @@ def pcg_launch_form(dev, stream, m, k, iterations, launches, one_reduction):
     (m = 0: the rotor-stator sector of the shared-geometry batches, its 3 coil currents
     U[-15, 15] A), k samples, one Newton iteration whose inner PCG is capped at `iterations`
     CG iterations (tolerance 1e-30, so every launch runs exactly that many), repeated
-    `launches` times on one plan.  The launch-shape autotuner is off (FG_PCG_TUNE=0: the default value ring, no
-    column cache), so the PCG launches are exactly these.  Reports the CUDA-event time per CG
+    `launches` times on one plan of the streamed form.  The launch-shape autotuner is off
+    (FG_PCG_TUNE=0: the default value ring, no column cache), so the PCG launches are exactly these.  Reports the CUDA-event time per CG
     iteration of each launch and the algorithmic bytes per CG iteration."""
     import torch
 
@@ -812,7 +840,7 @@ def pcg_launch_form(dev, stream, m, k, iterations, launches, one_reduction):
     else:
         model = meshes.annular_sector()
         currents = np.random.default_rng(5).uniform(-15.0, 15.0, size=(k, model.circuit_count))
-    plan = fg.Plan(model, one_reduction=one_reduction)
+    plan = fg.Plan(model, one_reduction=one_reduction, streamed=True)
     peak, source = peaks()
     cur = torch.tensor(currents, device=dev)
     out_a = torch.empty((k, plan.N), dtype=torch.float64, device=dev)
@@ -820,7 +848,7 @@ def pcg_launch_form(dev, stream, m, k, iterations, launches, one_reduction):
                                  linear_relative_tolerance=1e-30, adaptive_linear_tolerance=0,
                                  recover_nonconvergence=0)
     per_item = pcg_bytes_per_item_iteration(plan.rows, plan.nnz, 0, 0)
-    shared = 4.0 * plan.nnz + 4.0 * (plan.rows + 1)
+    shared = pcg_shared_bytes(plan.rows, plan.nnz)
     runs = []
     for _ in range(launches):
         torch.cuda.synchronize()
@@ -883,19 +911,20 @@ def planar_2m_form(dev, stream, flush, samples=4):
         ms = e0.elapsed_time(e1)
         t = p.last_timing()
         item_its = sum(i.linear_iterations for i in info)
+        form = pcg_form(p, k, kw.get("precision", 0))
         per_item = pcg_bytes_per_item_iteration(p.rows, p.nnz, kw.get("precision", 0),
-                                                kw.get("block_size", 0) if kw.get("preconditioner") else 0)
-        shared = 4.0 * p.nnz + 4.0 * (p.rows + 1)
+                                                kw.get("block_size", 0) if kw.get("preconditioner") else 0, form)
+        shared = pcg_shared_bytes(p.rows, p.nnz, form)
         gbs = (item_its * per_item + t.pcg_iterations * shared) / (t.pcg_ms / 1e3) / 1e9
         a, b1, b2, f = (out_a.cpu().numpy(), out_b1.cpu().numpy(), out_b2.cpu().numpy(), out_f.cpu().numpy())
         r = {"samples": k, "solves_per_s": k / (ms / 1e3), "seconds": ms / 1e3,
              "newton_iterations_per_item": float(np.mean([i.iterations for i in info])),
              "pcg_iterations_per_item": item_its / k, "pcg_ms": t.pcg_ms,
              "pcg_ms_per_cg_iteration": t.pcg_ms / max(1, t.pcg_iterations),
-             "pcg_gbs": gbs, "pcg_frac": gbs / peak,
+             "pcg_gbs": gbs, "pcg_frac": gbs / peak, "pcg_kernel": PCG_KERNELS[form],
              "mixed_fallbacks": int(t.mixed_fallbacks), "all_converged": all(i.status == 0 for i in info)}
         if name == "fp64_jacobi_k1":
-            per_it, src = traffic_per_cg_iteration("square1414_items1")
+            per_it, src = traffic_per_cg_iteration("square1414_items1", form)
             if per_it:
                 r["dram_traffic_per_cg_iteration"] = per_it
                 r["algorithmic_bytes_per_cg_iteration"] = per_item + shared
