@@ -191,56 +191,56 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
   {
     FG_GROUPS
     {
-    double v[2][IV] = {};
-    FG_STEPS
-    {
-      const int row = row_at(st), len = __ldg(a.row_len + row), e0 = off[st], W = off[st + 1] - e0;
-      const size_t base = position(st), ri = item_at(st);
-      const double zero[IV] = {};
-      for (int w = 0; w < W; ++w) {
-        // Places past the row's end: the row's own column with the value 0 (STREAM: -1).
-        const size_t pos = base + 32 * static_cast<size_t>(w);
-        if (lane % LR == 0)
-          column(e0 + w) = w < len ? __ldg(a.sell_col + pos) * KP : (STREAM ? -1 : row * KP);
-        if constexpr (!STREAM) {
-          if constexpr (SHARED) {
-            if (lane % LR == 0)
-              *stored(e0 + w) = w < len ? __ldg(vals + pos) : 0.0;
-          } else {
-            double vv[IV] = {};
-            if (w < len)
-              LoadStream<double, IV>(vals + pos * KP + item0, vv);
-            Store<double, IV>(stored(e0 + w), vv);
+      double v[2][IV] = {};
+      FG_STEPS
+      {
+        const int row = row_at(st), len = __ldg(a.row_len + row), e0 = off[st], W = off[st + 1] - e0;
+        const size_t base = position(st), ri = item_at(st);
+        const double zero[IV] = {};
+        for (int w = 0; w < W; ++w) {
+          // Places past the row's end: the row's own column with the value 0 (STREAM: -1).
+          const size_t pos = base + 32 * static_cast<size_t>(w);
+          if (lane % LR == 0)
+            column(e0 + w) = w < len ? __ldg(a.sell_col + pos) * KP : (STREAM ? -1 : row * KP);
+          if constexpr (!STREAM) {
+            if constexpr (SHARED) {
+              if (lane % LR == 0)
+                *stored(e0 + w) = w < len ? __ldg(vals + pos) : 0.0;
+            } else {
+              double vv[IV] = {};
+              if (w < len)
+                LoadStream<double, IV>(vals + pos * KP + item0, vv);
+              Store<double, IV>(stored(e0 + w), vv);
+            }
           }
+          Store<double, IV>(direction(e0 + w), zero);
         }
-        Store<double, IV>(direction(e0 + w), zero);
-      }
-      const double *src = static_cast<const double *>(a.use_inverse ? a.invd : a.diag);
-      if constexpr (SHARED) {
-        if (lane % LR == 0)
-          *vec(st, L::kInv) = __ldg(src + row);
-      } else {
-        double d[IV];
-        LoadRO<double, IV>(src + ri, d);
-        Store<double, IV>(vec(st, L::kInv), d);
-      }
-      Store<double, IV>(vec(st, L::kX), zero);
-      Store<double, IV>(vec(st, L::kP), zero);
-      double dd[IV], bb[IV];
-      Load<double, IV>(B + ri, bb);
-      LoadOperand<double, IV>(static_cast<const double *>(a.diag), static_cast<size_t>(row), a.diag_stride,
-                              a.diag_item, item0, dd);
+        const double *src = static_cast<const double *>(a.use_inverse ? a.invd : a.diag);
+        if constexpr (SHARED) {
+          if (lane % LR == 0)
+            *vec(st, L::kInv) = __ldg(src + row);
+        } else {
+          double d[IV];
+          LoadRO<double, IV>(src + ri, d);
+          Store<double, IV>(vec(st, L::kInv), d);
+        }
+        Store<double, IV>(vec(st, L::kX), zero);
+        Store<double, IV>(vec(st, L::kP), zero);
+        double dd[IV], bb[IV];
+        Load<double, IV>(B + ri, bb);
+        LoadOperand<double, IV>(static_cast<const double *>(a.diag), static_cast<size_t>(row), a.diag_stride,
+                                a.diag_item, item0, dd);
 #pragma unroll
-      for (int j = 0; j < IV; ++j)
-        if (on(j) && row < a.n) {
-          const double bj = bb[j], dj = dd[j];
-          const bool nonfinite = !isfinite(bj) || !isfinite(dj);
-          if (nonfinite || !(dj > 0.0))
-            v[0][j] = fmax(v[0][j], 2.0 * static_cast<double>(a.n - row) + (nonfinite ? 1.0 : 0.0));
-          v[1][j] = fmax(v[1][j], fabs(bj));
-        }
-    }
-    WarpPart<KP, IV, GV, 2, true>(v, gv * kPcgWarps + group_warp(gv), sm);
+        for (int j = 0; j < IV; ++j)
+          if (on(j) && row < a.n) {
+            const double bj = bb[j], dj = dd[j];
+            const bool nonfinite = !isfinite(bj) || !isfinite(dj);
+            if (nonfinite || !(dj > 0.0))
+              v[0][j] = fmax(v[0][j], 2.0 * static_cast<double>(a.n - row) + (nonfinite ? 1.0 : 0.0));
+            v[1][j] = fmax(v[1][j], fabs(bj));
+          }
+      }
+      WarpPart<KP, IV, GV, 2, true>(v, gv * kPcgWarps + group_warp(gv), sm);
     }
     if (!BarrierReduce<KP, GV, 2, true>(a, rank, ctas, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
           if (!ctl.active[it])
@@ -266,28 +266,28 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
   {
     FG_GROUPS
     {
-    double v[2][IV] = {};
-    FG_STEPS
-    {
-      double bb[IV], rv[IV], zv[IV];
-      Load<double, IV>(B + item_at(st), bb);
+      double v[2][IV] = {};
+      FG_STEPS
+      {
+        double bb[IV], rv[IV], zv[IV];
+        Load<double, IV>(B + item_at(st), bb);
 #pragma unroll
-      for (int j = 0; j < IV; ++j)
-        rv[j] = bb[j] / (ctl.scale[item0 + j] != 0.0 ? ctl.scale[item0 + j] : 1.0);
-      precond(st, rv, zv);
-      Store<double, IV>(vec(st, L::kR), rv);
-      send_z(z_buffer(0), st, zv);
+        for (int j = 0; j < IV; ++j)
+          rv[j] = bb[j] / (ctl.scale[item0 + j] != 0.0 ? ctl.scale[item0 + j] : 1.0);
+        precond(st, rv, zv);
+        Store<double, IV>(vec(st, L::kR), rv);
+        send_z(z_buffer(0), st, zv);
 #pragma unroll
-      for (int t = 1; t < 4; ++t)
-        reset_z(z_buffer(t), st);
+        for (int t = 1; t < 4; ++t)
+          reset_z(z_buffer(t), st);
 #pragma unroll
-      for (int j = 0; j < IV; ++j)
-        if (on(j)) {
-          v[0][j] += rv[j] * rv[j];
-          v[1][j] += rv[j] * zv[j];
-        }
-    }
-    WarpPart<KP, IV, GV, 2, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+        for (int j = 0; j < IV; ++j)
+          if (on(j)) {
+            v[0][j] += rv[j] * rv[j];
+            v[1][j] += rv[j] * zv[j];
+          }
+      }
+      WarpPart<KP, IV, GV, 2, false>(v, gv * kPcgWarps + group_warp(gv), sm);
     }
     if (!BarrierReduce<KP, GV, 2, false>(a, rank, ctas, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
           if (!ctl.active[it])
@@ -368,79 +368,79 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
         be[j] = ctl.beta[item0 + j];
       FG_GROUPS
       {
-      double v[1][IV] = {};
-      if (active & bits) {
-        FG_STEPS
-        {
-          const int e0 = off[st], W = off[st + 1] - e0;
-          const size_t pos = STREAM ? position(st) : 0;
-          double acc[IV] = {};
+        double v[1][IV] = {};
+        if (active & bits) {
+          FG_STEPS
+          {
+            const int e0 = off[st], W = off[st + 1] - e0;
+            const size_t pos = STREAM ? position(st) : 0;
+            double acc[IV] = {};
 #pragma unroll 1
-          for (int w0 = 0; w0 < W; w0 += U) {
-            double g[U][IV], vv[U][IV];
-            int c[U];
-            unsigned char *const en = resident_smem + entry0 + (e0 + w0) * L::kEntry;
+            for (int w0 = 0; w0 < W; w0 += U) {
+              double g[U][IV], vv[U][IV];
+              int c[U];
+              unsigned char *const en = resident_smem + entry0 + (e0 + w0) * L::kEntry;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              c[u] = -1;
-              if (w0 + u < W)
-                c[u] = *reinterpret_cast<const int32_t *>(en + u * L::kEntry + L::kColumn + rl * 4);
-            }
-            auto gather = [&] {
-#pragma unroll
-              for (int u = 0; u < U; ++u)
-                if (c[u] >= 0)
-                  LoadMessage<IV>(z + c[u] + item0, g[u]);
-            };
-            gather();
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (w0 + u < W)
-                value(pos, w0 + u, e0 + w0 + u, vv[u]);
-            auto missing = [&] {
-              bool m = false;
-#pragma unroll
-              for (int u = 0; u < U; ++u)
-                m = m || (c[u] >= 0 && Missing<IV>(g[u]));
-              return m;
-            };
-            if (missing()) { // z was sent before its owner's partial sums: rare
-              const unsigned long long t0 = GlobalTimer();
-              unsigned spin = 0;
-              do
-                gather();
-              while (missing() && PollAgain(a, spin, t0, sm));
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-              if (c[u] >= 0) {
-                double *const d = reinterpret_cast<double *>(en + u * L::kEntry + lane * IV * 8);
-                double pj[IV];
-                Load<double, IV>(d, pj);
-#pragma unroll
-                for (int j = 0; j < IV; ++j) {
-                  pj[j] = Fma(be[j], pj[j], g[u][j]);
-                  acc[j] = Fma(vv[u][j], pj[j], acc[j]);
-                }
-                Store<double, IV>(d, pj);
+              for (int u = 0; u < U; ++u) {
+                c[u] = -1;
+                if (w0 + u < W)
+                  c[u] = *reinterpret_cast<const int32_t *>(en + u * L::kEntry + L::kColumn + rl * 4);
               }
+              auto gather = [&] {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                  if (c[u] >= 0)
+                    LoadMessage<IV>(z + c[u] + item0, g[u]);
+              };
+              gather();
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+                if (w0 + u < W)
+                  value(pos, w0 + u, e0 + w0 + u, vv[u]);
+              auto missing = [&] {
+                bool m = false;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                  m = m || (c[u] >= 0 && Missing<IV>(g[u]));
+                return m;
+              };
+              if (missing()) { // z was sent before its owner's partial sums: rare
+                const unsigned long long t0 = GlobalTimer();
+                unsigned spin = 0;
+                do
+                  gather();
+                while (missing() && PollAgain(a, spin, t0, sm));
+              }
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+                if (c[u] >= 0) {
+                  double *const d = reinterpret_cast<double *>(en + u * L::kEntry + lane * IV * 8);
+                  double pj[IV];
+                  Load<double, IV>(d, pj);
+#pragma unroll
+                  for (int j = 0; j < IV; ++j) {
+                    pj[j] = Fma(be[j], pj[j], g[u][j]);
+                    acc[j] = Fma(vv[u][j], pj[j], acc[j]);
+                  }
+                  Store<double, IV>(d, pj);
+                }
+            }
+            // The row's own z = M^-1 r again: the very product its readers were sent.
+            double rv[IV], zr[IV], pv[IV];
+            Load<double, IV>(vec(st, L::kR), rv);
+            Load<double, IV>(vec(st, L::kP), pv);
+            precond(st, rv, zr);
+#pragma unroll
+            for (int j = 0; j < IV; ++j)
+              pv[j] = Fma(be[j], pv[j], zr[j]);
+            Store<double, IV>(vec(st, L::kP), pv);
+            Store<double, IV>(vec(st, L::kQ), acc);
+#pragma unroll
+            for (int j = 0; j < IV; ++j)
+              v[0][j] += pv[j] * acc[j];
           }
-          // The row's own z = M^-1 r again: the very product its readers were sent.
-          double rv[IV], zr[IV], pv[IV];
-          Load<double, IV>(vec(st, L::kR), rv);
-          Load<double, IV>(vec(st, L::kP), pv);
-          precond(st, rv, zr);
-#pragma unroll
-          for (int j = 0; j < IV; ++j)
-            pv[j] = Fma(be[j], pv[j], zr[j]);
-          Store<double, IV>(vec(st, L::kP), pv);
-          Store<double, IV>(vec(st, L::kQ), acc);
-#pragma unroll
-          for (int j = 0; j < IV; ++j)
-            v[0][j] += pv[j] * acc[j];
         }
-      }
-      WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+        WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
       }
     }
     if (warp == 0) {
@@ -486,32 +486,32 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
       }
       FG_GROUPS
       {
-      double v[2][IV] = {};
-      if (mine)
-        FG_STEPS
-        {
-          double xv[IV], rv[IV], qv[IV], pv[IV], zv[IV];
-          Load<double, IV>(vec(st, L::kR), rv);
-          Load<double, IV>(vec(st, L::kQ), qv);
-          Load<double, IV>(vec(st, L::kX), xv);
-          Load<double, IV>(vec(st, L::kP), pv);
+        double v[2][IV] = {};
+        if (mine)
+          FG_STEPS
+          {
+            double xv[IV], rv[IV], qv[IV], pv[IV], zv[IV];
+            Load<double, IV>(vec(st, L::kR), rv);
+            Load<double, IV>(vec(st, L::kQ), qv);
+            Load<double, IV>(vec(st, L::kX), xv);
+            Load<double, IV>(vec(st, L::kP), pv);
 #pragma unroll
-          for (int j = 0; j < IV; ++j)
-            if (act[j]) {
-              rv[j] = rv[j] - al[j] * qv[j];
-              xv[j] = xv[j] + al[j] * pv[j];
+            for (int j = 0; j < IV; ++j)
+              if (act[j]) {
+                rv[j] = rv[j] - al[j] * qv[j];
+                xv[j] = xv[j] + al[j] * pv[j];
+              }
+            precond(st, rv, zv);
+            send_z(zn, st, zv);
+            Store<double, IV>(vec(st, L::kX), xv);
+            Store<double, IV>(vec(st, L::kR), rv);
+#pragma unroll
+            for (int j = 0; j < IV; ++j) {
+              v[0][j] += rv[j] * rv[j];
+              v[1][j] += rv[j] * zv[j];
             }
-          precond(st, rv, zv);
-          send_z(zn, st, zv);
-          Store<double, IV>(vec(st, L::kX), xv);
-          Store<double, IV>(vec(st, L::kR), rv);
-#pragma unroll
-          for (int j = 0; j < IV; ++j) {
-            v[0][j] += rv[j] * rv[j];
-            v[1][j] += rv[j] * zv[j];
           }
-        }
-      WarpPart<KP, IV, GV, 2, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+        WarpPart<KP, IV, GV, 2, false>(v, gv * kPcgWarps + group_warp(gv), sm);
       }
     }
     // While the sums travel: reset the z of this iteration
@@ -589,21 +589,21 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
           return;
         FG_GROUPS
         {
-        double v[1][IV] = {};
-        FG_STEPS
-        {
-          double rv[IV], t[IV];
-          true_residual(st, t);
-          Load<double, IV>(vec(st, L::kR), rv);
+          double v[1][IV] = {};
+          FG_STEPS
+          {
+            double rv[IV], t[IV];
+            true_residual(st, t);
+            Load<double, IV>(vec(st, L::kR), rv);
 #pragma unroll
-          for (int j = 0; j < IV; ++j)
-            if (on(j) && ctl.flag[item0 + j] == 1) {
-              rv[j] = t[j];
-              v[0][j] += t[j] * t[j];
-            }
-          Store<double, IV>(vec(st, L::kR), rv);
-        }
-        WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+            for (int j = 0; j < IV; ++j)
+              if (on(j) && ctl.flag[item0 + j] == 1) {
+                rv[j] = t[j];
+                v[0][j] += t[j] * t[j];
+              }
+            Store<double, IV>(vec(st, L::kR), rv);
+          }
+          WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
         }
         if (!BarrierReduce<KP, GV, 1, false>(a, rank, ctas, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
               if (!ctl.active[it] || ctl.flag[it] != 1)
@@ -621,32 +621,32 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
       }
       FG_GROUPS
       {
-      double v[2][IV] = {};
-      FG_STEPS
-      {
-        double xv[IV], rv[IV], zv[IV];
-        Load<double, IV>(vec(st, L::kX), xv);
-        Load<double, IV>(vec(st, L::kR), rv);
-        precond(st, rv, zv);
-        bool restart = false;
+        double v[2][IV] = {};
+        FG_STEPS
+        {
+          double xv[IV], rv[IV], zv[IV];
+          Load<double, IV>(vec(st, L::kX), xv);
+          Load<double, IV>(vec(st, L::kR), rv);
+          precond(st, rv, zv);
+          bool restart = false;
 #pragma unroll
-        for (int j = 0; j < IV; ++j) {
-          const int f = on(j) ? ctl.flag[item0 + j] : 0;
-          if (f == 2) {
-            xv[j] = xv[j] * ctl.scale[item0 + j];
-            if (!isfinite(xv[j]))
-              v[1][j] += 1.0;
+          for (int j = 0; j < IV; ++j) {
+            const int f = on(j) ? ctl.flag[item0 + j] : 0;
+            if (f == 2) {
+              xv[j] = xv[j] * ctl.scale[item0 + j];
+              if (!isfinite(xv[j]))
+                v[1][j] += 1.0;
+            }
+            if (f == 3) {
+              v[0][j] += rv[j] * zv[j];
+              restart = true;
+            }
           }
-          if (f == 3) {
-            v[0][j] += rv[j] * zv[j];
-            restart = true;
-          }
+          Store<double, IV>(vec(st, L::kX), xv);
+          if (restart) // items that go on keep r, so their z is the same product again
+            send_z(zn, st, zv);
         }
-        Store<double, IV>(vec(st, L::kX), xv);
-        if (restart) // items that go on keep r, so their z is the same product again
-          send_z(zn, st, zv);
-      }
-      WarpPart<KP, IV, GV, 2, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+        WarpPart<KP, IV, GV, 2, false>(v, gv * kPcgWarps + group_warp(gv), sm);
       }
       if (!BarrierReduce<KP, GV, 2, false>(a, rank, ctas, G, sm, epoch, buf, [&](int it, const double (&sum)[2]) {
             if (!ctl.active[it])
@@ -683,17 +683,17 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
     {
       FG_GROUPS
       {
-      double v[1][IV] = {};
-      FG_STEPS
-      {
-        double t[IV];
-        true_residual(st, t);
+        double v[1][IV] = {};
+        FG_STEPS
+        {
+          double t[IV];
+          true_residual(st, t);
 #pragma unroll
-        for (int j = 0; j < IV; ++j)
-          if (on(j))
-            v[0][j] += t[j] * t[j];
-      }
-      WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+          for (int j = 0; j < IV; ++j)
+            if (on(j))
+              v[0][j] += t[j] * t[j];
+        }
+        WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
       }
       if (!BarrierReduce<KP, GV, 1, false>(a, rank, ctas, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
             if (!ctl.active[it])
@@ -710,21 +710,21 @@ __global__ void __launch_bounds__(kPcgThreads, 1) PcgResidentStepsKernel(PcgArgs
     }
     FG_GROUPS
     {
-    double v[1][IV] = {};
-    FG_STEPS
-    {
-      double xv[IV];
-      Load<double, IV>(vec(st, L::kX), xv);
+      double v[1][IV] = {};
+      FG_STEPS
+      {
+        double xv[IV];
+        Load<double, IV>(vec(st, L::kX), xv);
 #pragma unroll
-      for (int j = 0; j < IV; ++j)
-        if (on(j)) {
-          xv[j] = xv[j] * ctl.scale[item0 + j];
-          if (!isfinite(xv[j]))
-            v[0][j] += 1.0;
-        }
-      Store<double, IV>(vec(st, L::kX), xv);
-    }
-    WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
+        for (int j = 0; j < IV; ++j)
+          if (on(j)) {
+            xv[j] = xv[j] * ctl.scale[item0 + j];
+            if (!isfinite(xv[j]))
+              v[0][j] += 1.0;
+          }
+        Store<double, IV>(vec(st, L::kX), xv);
+      }
+      WarpPart<KP, IV, GV, 1, false>(v, gv * kPcgWarps + group_warp(gv), sm);
     }
     if (!BarrierReduce<KP, GV, 1, false>(a, rank, ctas, G, sm, epoch, buf, [&](int it, const double (&sum)[1]) {
           if (!ctl.active[it])
