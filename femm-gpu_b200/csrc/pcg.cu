@@ -178,10 +178,13 @@ size_t PcgPartialsDoubles(int kp, int grid)
 {
   // Double-buffered sums of the barrier-based reductions, then eight mailbox buffers of two sums
   // per item and row group and a line of results per CTA (pcg_resident.cuh); or the streamed
-  // kernels' buffers (at most three sums of 32 items).
+  // kernels' buffers (at most three sums of 32 items).  A mailbox buffer is counted as 64 KB at
+  // least, more than narrow launches use: with a tighter buffer a plan's arrays lie at other
+  // addresses, and how far a polled line is from the SMs that poll it depends on its address
+  // (4,225 rows, one item: 4.64 and 4.72 ms a solve).
   const size_t k = static_cast<size_t>(kp), g = static_cast<size_t>(grid);
-  const size_t line = std::max<size_t>(2 * k, 16);
-  return std::max<size_t>(4 * k * g + 8 * (2 * k * g + g * line), 2 * 96 * g);
+  const size_t sums = std::max<size_t>(2 * k * g, 8192), line = std::max<size_t>(2 * k, 16);
+  return std::max<size_t>(4 * k * g + 8 * (sums + g * line), 2 * 96 * g);
 }
 
 namespace
