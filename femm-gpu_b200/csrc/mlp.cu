@@ -133,8 +133,9 @@ __device__ __forceinline__ void Stage(float *smem, const float *X, int rs, int k
 // launch, of L2 and of each thread's chain -- not FP32 rate.  16 x 32 tiles give a 256 x 256
 // output 128 CTAs; a slab of the inner dimension up to 256 is staged at once, every one of 16
 // warps multiplies its own 16th of it with 4 x 4 outputs per lane (16 FMAs from two 16-byte
-// shared-memory reads), and the 16 partial tiles are added in warp order.  Measured (B200):
-// loss and gradient of a 4-256-256-64 network at batch 256 through host buffers 318 -> 155 us (two thirds of the rest are copies and the fresh host array).
+// shared-memory reads), and the 16 partial tiles are added in warp order.  Measured (B200): loss
+// and gradient of a 4-256-256-64 network at batch 256 through host buffers 319 -> 111 us, six
+// launches of about 5 us and copies.
 //
 // A short inner dimension (the first layer, narrow networks) has no work for 16 warps: with R > 1
 // they take R row tiles instead (RowTiles).  Where R is used, sums and their order are those of

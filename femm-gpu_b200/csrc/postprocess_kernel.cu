@@ -93,7 +93,7 @@ __device__ void Corner(const PostprocessDevice &p, const CornerStencil &c, const
 // mask has a gradient (some hundred elements); the products with B are taken everywhere, so
 // that a field that is not finite still shows in the sums.  With four items together, force,
 // probes and the results' way to the host in one launch: 19.5 us from cold caches, against 14.4 +
-// 5.4 us and a copy; the whole call 58 -> 35 us (32 items), 36 -> 22 us (one).
+// 5.4 us and a copy; the whole call 57.6 -> 34.4 us (32 items), 36 -> 22 us (one).
 template <int IT> __device__ void ForceCta(const PostprocessDevice &p, int cta, int group)
 {
   __shared__ double scratch[kThreads / 32][3 * IT];
